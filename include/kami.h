@@ -253,10 +253,11 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type,
  * problem by its warp partition; (FP16 / BF16 inputs) the tcgen05 kernel,
  * which issues each problem's MMAs from one thread into tensor memory while
  * loader and epilogue warps stream the operands and C; and (FP64 inputs) the
- * staged DMMA kernel, whose loader warps stream K chunks into shared memory
- * while fourteen compute warps share each problem's C.  The tcgen05 kernel
- * is the default for FP16 / BF16, the staged kernel for FP64 (the warp-grid
- * kernel when problems of at most 32 x 32 carry most of the bytes);
+ * ring DMMA kernel, whose copying warps stream whole problems, or K chunks of
+ * the large ones, through a shared-memory ring to sixteen computing warps.
+ * The tcgen05 kernel is the default for FP16 / BF16, the ring kernel for FP64
+ * (the warp-grid kernel for plans below 10 MB when problems of at most
+ * 32 x 32 carry most of the bytes);
  * KAMI_PLAN_MMA_SYNC / KAMI_PLAN_TCGEN05 / KAMI_PLAN_STAGED force one.  With
  * flags & KAMI_PLAN_AUTOTUNE the plan first measures every valid partition
  * per 16-rounded shape bucket on this device (cached per process) instead of
@@ -288,7 +289,7 @@ int kami_gemm_grouped_run(const kami_grouped_plan *plan, const void *A, const vo
  * out[3] = FLOPs, out[4] = bytes moved, out[5..12] = problems per partition
  * of the mma.sync kernel (0-2: 1D/2D warp grids, 3-6: 3D warp grids with K
  * depth, 7: one warp per problem), out[13] = kernel (0 mma.sync, 1 tcgen05,
- * 2 staged FP64 DMMA),
+ * 2 FP64 ring),
  * out[14] / out[15] = problems on M = 64 / M = 128 tcgen05 MMAs. */
 int kami_gemm_grouped_plan_info(const kami_grouped_plan *plan, int64_t out[16]);
 int kami_gemm_grouped_plan_destroy(kami_grouped_plan *plan);

@@ -291,7 +291,7 @@ class GroupedPlan:
     shapes: sequence of (M, N, K).  Problems are packed back to back in the
     A, B and C buffers (A_i M x K, B_i N x K, C_i M x N, row-major) unless
     explicit element offsets are given.  kernel: None (the library's choice:
-    tcgen05 for FP16 / BF16, staged DMMA for FP64, measured against mma.sync
+    tcgen05 for FP16 / BF16, the ring kernel for FP64, measured against mma.sync
     when autotuned), "mma_sync", "tcgen05" or "staged" (KAMI_PLAN_MMA_SYNC /
     KAMI_PLAN_TCGEN05 / KAMI_PLAN_STAGED)."""
 

@@ -463,11 +463,11 @@ struct kami_grouped_plan
 {
     int in_type, out_type, count, ctas, smem;
     int kernel = 0; // 0: mma.sync warp grids (grouped_kernel), 1: tcgen05 (grouped_tc05_kernel),
-                    // 2: staged FP64 DMMA (grouped_f64_kernel)
+                    // 2: FP64 ring (f64_ring_kernel)
     int tc_m64 = 0, tc_m128 = 0; // tcgen05 plans: problems on M = 64 / M = 128 MMAs
     bool packed = false;         // tcgen05 plans: some work item holds several problems
     int small_begin = 0, small_end = 0; // desc range of single-warp problems
-    GroupedDesc *d_desc = nullptr;
+    void *d_desc = nullptr; // GroupedDesc per problem; chunk descriptors for FP64 ring plans
     int *d_begin = nullptr;
     int cfg_hist[kCfgs] = {0};
     int64_t flops = 0, bytes = 0;
@@ -540,7 +540,7 @@ static int launch_grouped(const kami_grouped_plan *plan, const void *A, const vo
                           double beta, int num_iter, cudaStream_t s)
 {
     GroupedParams p{};
-    p.desc = plan->d_desc;
+    p.desc = reinterpret_cast<const GroupedDesc *>(plan->d_desc);
     p.cta_begin = plan->d_begin;
     p.A = A;
     p.B = B;
@@ -554,7 +554,7 @@ static int launch_grouped(const kami_grouped_plan *plan, const void *A, const vo
     if (plan->kernel == 1)
         return grouped_tc05_launch(p, plan->in_type == KAMI_BF16, plan->packed, plan->ctas, s);
     if (plan->kernel == 2)
-        return grouped_f64s_launch(p, plan->ctas, s);
+        return grouped_f64s_launch(p, plan->d_desc, plan->ctas, s);
     void *args[] = {&p};
     cudaError_t e = cudaLaunchKernel(grouped_fn(plan->in_type), dim3(plan->ctas), dim3(kThreads), args,
                                      (size_t)plan->smem, s);
@@ -577,7 +577,7 @@ static int free_plan(kami_grouped_plan *pl)
 
 // Build descriptors + LPT schedule for `count` problems (host arrays) with
 // the given partitions and upload them.  kernel 1 (FP16 / BF16 only) is the
-// tcgen05 kernel, kernel 2 (FP64 only) the staged DMMA kernel: every problem
+// tcgen05 kernel, kernel 2 (FP64 only) the ring kernel: every problem
 // goes through their CTA pipelines (no single-warp problems); the tcgen05
 // kernel's cost model is its bytes plus a fixed per-problem latency.
 static int build_plan(int in_type, int out_type, int count, const int *M, const int *N, const int *K,
@@ -695,24 +695,24 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
             pl->packed = pl->packed || it.size() > 1;
         }
     }
-    else
-        for (int i : order)
-            items.push_back({i});
-    if (tc)
-        for (const auto &it : items)
-        {
-            int mt = 0;
-            for (int i : it)
-                mt += M[i];
-            (mt <= 64 ? pl->tc_m64 : pl->tc_m128) += (int)it.size();
-        }
-    std::vector<double> icost(items.size(), 2048.0);
-    std::vector<int> iorder(items.size());
-    for (size_t t = 0; t < items.size(); ++t)
+    // members of item t: without packing, problem t alone
+    const bool packing = tc && pack;
+    const int nitems = packing ? (int)items.size() : count;
+    auto first_of = [&](int t) { return packing ? items[t].data() : &order[t]; };
+    auto size_of = [&](int t) { return packing ? (int)items[t].size() : 1; };
+    std::vector<double> icost(nitems, 2048.0);
+    std::vector<int> iorder(nitems);
+    for (int t = 0; t < nitems; ++t)
     {
-        for (int i : items[t])
-            icost[t] += cost[i] - 2048.0;
-        iorder[t] = (int)t;
+        int mt = 0;
+        for (const int *i = first_of(t); i != first_of(t) + size_of(t); ++i)
+        {
+            icost[t] += cost[*i] - 2048.0;
+            mt += M[*i];
+        }
+        if (tc)
+            (mt <= 64 ? pl->tc_m64 : pl->tc_m128) += size_of(t);
+        iorder[t] = t;
     }
     std::stable_sort(iorder.begin(), iorder.end(), [&](int a, int b) { return icost[a] > icost[b]; });
     typedef std::pair<double, int> Load;
@@ -723,7 +723,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     std::vector<int> smalls;
     for (int t : iorder)
     {
-        const int i = items[t][0];
+        const int i = *first_of(t);
         if (cfg[i] == 7 && kernel == 0)
         {
             smalls.push_back(i); // longest first, spread over all warps round-robin
@@ -737,7 +737,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     std::vector<GroupedDesc> desc;
     desc.reserve(count);
     std::vector<int> begin(ctas + 1, 0);
-    for (int c = 0; c < ctas; ++c)
+    for (int c = 0; c < ctas && !staged; ++c)
     {
         begin[c] = (int)desc.size();
         for (int t : lists[c])
@@ -745,16 +745,21 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
             // tcgen05 plans: the item's extent in every member (see item_at in
             // grouped_tc05.cu): count | Mt << 3 | (Nt / 16) << 11 | Kt << 15
             int mt = 0, nt = 0, kt = 0;
-            for (int i : items[t])
+            const int *members = first_of(t), *members_end = members + size_of(t);
+            for (const int *m = members; m != members_end; ++m)
             {
+                const int i = *m;
                 mt = std::max(mt, (pk[i] & 0xff) + M[i]);
                 nt = std::max(nt, ((pk[i] >> 8) & 0xff) + ((N[i] + 15) & ~15));
                 kt = std::max(kt, K[i]);
             }
-            const int ext = tc ? (int)items[t].size() | (mt << 3) | ((nt / 16) << 11) | (kt << 15) : 0;
-            for (int i : items[t])
+            const int ext = tc ? size_of(t) | (mt << 3) | ((nt / 16) << 11) | (kt << 15) : 0;
+            for (const int *m = members; m != members_end; ++m)
+            {
+                const int i = *m;
                 desc.push_back(GroupedDesc{M[i], N[i], K[i], tc ? pk[i] : cfg[i], ao[i], bo[i], co[i],
                                            lda ? lda[i] : K[i], ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i], ext});
+            }
         }
     }
     begin[ctas] = (int)desc.size();
@@ -763,14 +768,19 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
         desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], lda ? lda[i] : K[i],
                                    ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i], 0});
     pl->small_end = (int)desc.size();
-    if ((e = cudaMalloc(&pl->d_desc, sizeof(GroupedDesc) * std::max(count, 1))) != cudaSuccess ||
+    // FP64 ring plans: the chunks of every CTA's problems instead of the problems
+    std::vector<char> chunks;
+    if (staged)
+        f64_ring_schedule(lists, M, N, K, ao, bo, co, &chunks, &begin);
+    const void *src = staged ? (const void *)chunks.data() : (const void *)desc.data();
+    const size_t src_bytes = staged ? chunks.size() : sizeof(GroupedDesc) * desc.size();
+    if ((e = cudaMalloc(&pl->d_desc, std::max(src_bytes, (size_t)16))) != cudaSuccess ||
         (e = cudaMalloc(&pl->d_begin, sizeof(int) * (ctas + 1))) != cudaSuccess)
     {
         free_plan(pl);
         return cuda_fail(e, "cudaMalloc(grouped plan)");
     }
-    if ((e = cudaMemcpy(pl->d_desc, desc.data(), sizeof(GroupedDesc) * count, cudaMemcpyHostToDevice)) !=
-            cudaSuccess ||
+    if ((e = cudaMemcpy(pl->d_desc, src, src_bytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(pl->d_begin, begin.data(), sizeof(int) * (ctas + 1), cudaMemcpyHostToDevice)) != cudaSuccess)
     {
         free_plan(pl);
@@ -854,6 +864,8 @@ int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream)
     if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.B) & 15) ||
         (reinterpret_cast<uintptr_t>(g.C) & 15))
         return fail(KAMI_ERR_UNSUPPORTED, "no kernel for this shape with unaligned buffers");
+    if (in_type == KAMI_F64)
+        return f64_ring_launch(g, stream);
     static std::mutex mu;
     static std::map<std::vector<int64_t>, kami_grouped_plan *> cache;
     int dev = 0;
@@ -879,7 +891,7 @@ int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream)
             co[i] = (int64_t)i * g.sC;
         }
         int st = build_plan(in_type, g.out_type, n, vm.data(), vn.data(), vk.data(), ao.data(), bo.data(), co.data(),
-                            vc.data(), &pl, la.data(), lb.data(), lc.data(), in_type == KAMI_F64 ? 2 : 1);
+                            vc.data(), &pl, la.data(), lb.data(), lc.data(), 1);
         if (st)
             return st;
         std::lock_guard<std::mutex> lk(mu);
@@ -1004,13 +1016,13 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
         }
     }
     // the kernel besides the warp-grid one: tcgen05 for 16-bit inputs, the
-    // staged DMMA kernel for FP64
+    // ring kernel for FP64
     const int alt = in_type == KAMI_F64 ? 2 : 1;
-    // FP64 without a measurement: the staged kernel, unless problems of at
-    // most 32 x 32 carry most of the bytes -- its fourteen compute warps pay
-    // a fixed cost per problem that the warp-grid kernel's one-warp path for
-    // such problems does not (20000 problems of 32^3: 0.21 ms staged, 0.15
-    // warp grids; the uneven 8..128 mix: 0.36 against 0.81)
+    // FP64 without a measurement: the ring kernel, except that a plan of less
+    // than 10 MB with most of its bytes in problems of at most 32 x 32 keeps the
+    // warp-grid kernel it has always reported (measured, the ring is ahead from
+    // 1000 problems on: 1000 of 8..32 5.0 against 7.4 us, 20000 of 32^3 78
+    // against 146; 1000 of 8^3 4.5 against 4.0)
     bool tiny_mix = false;
     if (in_type == KAMI_F64 && !force_st && !tune)
     {
@@ -1022,7 +1034,7 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
             if (M[i] <= 32 && N[i] <= 32)
                 tiny += by;
         }
-        tiny_mix = tiny > 0.6 * all;
+        tiny_mix = tiny > 0.6 * all && all * 8 < 10e6;
     }
     if (force_mma || tiny_mix)
         return build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), plan);

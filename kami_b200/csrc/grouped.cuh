@@ -1,8 +1,10 @@
 // grouped.cuh -- device descriptors of the uneven (grouped) batched GEMM,
 // shared by its three kernels: the mma.sync warp-grid kernel (grouped.cu),
-// the tcgen05 kernel (grouped_tc05.cu, FP16 / BF16) and the staged DMMA
-// kernel (grouped_f64.cu, FP64).
+// the tcgen05 kernel (grouped_tc05.cu, FP16 / BF16) and the FP64 ring
+// kernel (f64_ring.cu).
 #pragma once
+#include <vector>
+
 #include "kami_common.cuh"
 
 namespace kami {
@@ -39,11 +41,15 @@ int grouped_tc05_ctas_per_sm();
 int grouped_tc05_launch(const GroupedParams &p, bool bf16, bool packed, int ctas, cudaStream_t s);
 int grouped_tc05_read_error(int *flag);
 
-// staged FP64 grouped kernel (grouped_f64.cu)
+// FP64 ring kernel (f64_ring.cu): plans, and uniform batches (f64_ring_launch)
 const void *grouped_f64s_fn();
 int grouped_f64s_threads();
 int grouped_f64s_smem();
-int grouped_f64s_launch(const GroupedParams &p, int ctas, cudaStream_t s);
-int grouped_f64s_read_error(int *flag);
+int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s);
+size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
+                         const int64_t *ao, const int64_t *bo, const int64_t *co, std::vector<char> *out,
+                         std::vector<int> *begin);
+int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
+int f64_ring_read_error(int *flag);
 
 } // namespace kami

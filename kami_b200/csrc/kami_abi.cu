@@ -1,6 +1,7 @@
 // kami_abi.cu -- the C ABI of libkami_b200.so: argument validation, kernel
 // selection (the reference's compile-time -D knobs become run-time
 // arguments), launch configuration and error reporting.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -12,15 +13,14 @@
 
 namespace kami {
 
-int f64_stream_launch(const GemmArgs &g, cudaStream_t s);
-int f64s_read_error(int *flag);
 int grouped_tc05_read_error(int *flag);
 int spgemm_read_error(int *flag);
-int grouped_f64s_read_error(int *flag);
+int f64_ring_read_error(int *flag);
 int spmm_tc05_read_error(int *flag);
 int spgemm_tc05_read_error(int *flag);
 int split_read_error(int *flag);
 int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream);
+int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
 
 static thread_local char g_err[512] = "no error";
 
@@ -252,16 +252,14 @@ int kami_device_status(int *code)
     int st = tc05_read_error(code);
     if (st)
         return st;
-    int c2 = 0, c3 = 0, c4 = 0, c5 = 0, c6 = 0, c7 = 0;
+    int c2 = 0, c4 = 0, c5 = 0, c6 = 0, c7 = 0;
     if ((st = split_read_error(&c2)))
-        return st;
-    if ((st = f64s_read_error(&c3)))
         return st;
     if ((st = grouped_tc05_read_error(&c4)))
         return st;
     if ((st = spgemm_read_error(&c5)))
         return st;
-    if ((st = grouped_f64s_read_error(&c6)))
+    if ((st = f64_ring_read_error(&c6)))
         return st;
     if ((st = spmm_tc05_read_error(&c7)))
         return st;
@@ -270,8 +268,6 @@ int kami_device_status(int *code)
         return st;
     if (!*code)
         *code = c2;
-    if (!*code)
-        *code = c3;
     if (!*code)
         *code = c4;
     if (!*code)
@@ -446,16 +442,23 @@ int gemm_batched_hinted(kami_dtype_t in_type, kami_dtype_t out_type, kami_partit
             return st;
     }
 
-    // streamed FP64 problems up to 64^3 (the batched FP64 programs' regime):
-    // the persistent kernel that overlaps each problem's loads with the
-    // DMMAs of the previous ones, when the choice is left to the library and
-    // there are at least two problems per SM (148 SMs)
+    // streamed FP64 problems: the ring kernel, when the choice is left to the
+    // library.  The per-problem kernel keeps what it holds in a compiled block
+    // without much padding and without a persistent kernel's start-up: up to
+    // 16^3 (400 MB of 16^3 58.6 us against 72, 2 MB of 8^3 2.2 against 3.6), and
+    // up to 32^3 below 32 MB or with strided rows (16 MB of 32^3 5.4 us against
+    // 6.3, 100 MB 24.6 against 21; strided, which the ring copies row by row,
+    // 150 MB 34 against 47).  Elsewhere the ring is ahead, from 1.1x at
+    // 64^3 to 5x where a 64^3 block is mostly padding (40 x 24 x 32).
     if (in_type == KAMI_F64 && variant == KAMI_VARIANT_AUTO && partition == KAMI_PARTITION_AUTO && P == 0 &&
-        alloc_warps == 0 && num_iter <= 4 && batch >= 296)
+        alloc_warps == 0 && num_iter <= 4 && M <= 64 && N <= 64 && K <= 64 && a_layout == KAMI_A_ROW_MK &&
+        b_layout == KAMI_B_REF_NK && lda <= 0x7fffffff && ldb <= 0x7fffffff && ldc <= 0x7fffffff)
     {
-        st = f64_stream_launch(g, s);
-        if (st != KAMI_ERR_UNSUPPORTED)
-            return st;
+        const int largest = std::max(M, std::max(N, K));
+        const bool packed = (lda == K || M == 1) && (ldb == K || N == 1);
+        const double bytes = 8.0 * batch * ((double)(M + N) * K + (double)M * N);
+        if (largest > 32 || (largest > 16 && packed && bytes >= 32e6))
+            return f64_ring_launch(g, s);
     }
 
     const MmaInstance *inst = nullptr;
