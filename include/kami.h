@@ -251,8 +251,8 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type,
  * descriptors and a longest-first schedule over persistent CTAs.  Three
  * kernels run a plan: the mma.sync kernel, whose eight warps split each
  * problem by its warp partition; (FP16 / BF16 inputs) the tcgen05 kernel,
- * which issues each problem's MMAs from one thread into tensor memory while
- * loader and epilogue warps stream the operands and C; and (FP64 inputs) the
+ * whose CTAs run four pipelines of copying, MMA-issuing and storing warps side
+ * by side; and (FP64 inputs) the
  * ring DMMA kernel, whose copying warps stream whole problems, or K chunks of
  * the large ones, through a shared-memory ring to sixteen computing warps.
  * The tcgen05 kernel is the default for FP16 / BF16, the ring kernel for FP64
@@ -270,12 +270,9 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type,
 #define KAMI_PLAN_MMA_SYNC 2
 #define KAMI_PLAN_TCGEN05 4
 #define KAMI_PLAN_STAGED 8
-/* With this flag a tcgen05 plan puts up to four problems of at most 64 rows
- * and 64 columns (rounded to 16) in one work item -- their A rows stacked in
- * one 128-row tile, their B rows in another, C on the accumulator's diagonal
- * -- so one chain of MMAs and one accumulator hand-off serve them all.  Off
- * by default: on the 20000-problem 8..128 mix it measured slower (0.104 ms
- * against 0.096 ms one problem per item). */
+/* Asked tcgen05 plans to put several small problems in one work item.  Accepted
+ * and without effect: one problem per item is faster (20000 problems of 8..128:
+ * 0.066 ms; packed, in the kernel that did so, 0.104). */
 #define KAMI_PLAN_PACK 16
 typedef struct kami_grouped_plan kami_grouped_plan;
 
@@ -290,7 +287,7 @@ int kami_gemm_grouped_run(const kami_grouped_plan *plan, const void *A, const vo
  * of the mma.sync kernel (0-2: 1D/2D warp grids, 3-6: 3D warp grids with K
  * depth, 7: one warp per problem), out[13] = kernel (0 mma.sync, 1 tcgen05,
  * 2 FP64 ring),
- * out[14] / out[15] = problems on M = 64 / M = 128 tcgen05 MMAs. */
+ * out[14] / out[15] = problems on M = 64 / M = 128 tcgen05 MMAs (all on M = 128). */
 int kami_gemm_grouped_plan_info(const kami_grouped_plan *plan, int64_t out[16]);
 int kami_gemm_grouped_plan_destroy(kami_grouped_plan *plan);
 

@@ -293,7 +293,8 @@ class GroupedPlan:
     explicit element offsets are given.  kernel: None (the library's choice:
     tcgen05 for FP16 / BF16, the ring kernel for FP64, measured against mma.sync
     when autotuned), "mma_sync", "tcgen05" or "staged" (KAMI_PLAN_MMA_SYNC /
-    KAMI_PLAN_TCGEN05 / KAMI_PLAN_STAGED)."""
+    KAMI_PLAN_TCGEN05 / KAMI_PLAN_STAGED).  pack (KAMI_PLAN_PACK) is accepted
+    and has no effect."""
 
     def __init__(self, shapes, dtype=torch.float16, out_dtype=None, *, autotune=False, offsets=None, kernel=None,
                  pack=False):

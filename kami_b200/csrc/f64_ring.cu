@@ -57,6 +57,7 @@
 
 #include "grouped.cuh"
 #include "kami_common.cuh"
+#include "ring.cuh"
 #include "tc05_ptx.cuh"
 
 namespace kami {
@@ -69,14 +70,14 @@ __device__ int g_f64r_error = 0;
 
 namespace {
 
+using namespace ring;
+
 constexpr int kWarps = 16;                  // computing warps
 constexpr int kCopyWarps = 4;               // warps kWarps .. copy
 constexpr int kThreads = (kWarps + kCopyWarps) * 32;
-constexpr int kRecs = 32;                   // chunks in flight at most
 constexpr int kRing = 224 * 1024;           // bytes of staged operands
 constexpr int kWholeMax = 72 * 1024;        // bytes of a part copied whole: three fit the ring
 constexpr int kGroupMax = 16 * 1024;        // bytes of a part of several problems
-constexpr int kAhead = 64 * 1024;           // bytes in flight, the chunk that passes it included
 constexpr int kChunk = 64;                  // k values of a chunk at most (128 rows: three chunks fit the ring)
 
 struct __align__(16) Rec
@@ -93,21 +94,14 @@ constexpr int kSmem = kRing + kRecs * (int)sizeof(Rec) + 2 * kRecs * 8 + 128;
 static_assert(kSmem <= 227 * 1024, "f64 ring kernel: shared memory");
 
 // A chunk as the copying warps take it: the record (its addresses relative to
-// the ring), where it comes from, and what has to come before it: the last
-// chunk of its CTA that has to be done with before the bytes and the record
-// may be written, and the last one that has to have landed.  Bulk copies in
-// flight share the SM's bandwidth, so more of them than latency asks for only
-// delay the oldest: with the whole ring asked for at once the first chunk lands
-// with the last (64^3 x 610: 23.2 us, 20.0 with kAhead), and 32^3 x 65536 takes
-// 290 us instead of 257.
+// the ring), where it comes from, and what has to come before it (ring.cuh).
 struct __align__(16) ChunkDesc
 {
     Rec r;
     int64_t a_off, b_off; // elements
     uint16_t na, nb;      // rows of A and B
     int ld;               // 0: copied whole; a plan's row stride (a uniform batch has its own two)
-    int dep;              // chunk of the CTA that must be done with first
-    int land;             // chunk that must have landed first
+    int dep, land;
 };
 static_assert(sizeof(ChunkDesc) == 64, "chunk descriptor");
 
@@ -254,7 +248,6 @@ __device__ __forceinline__ void store_tile(double *Cb, int M, int N, int ldc, bo
 
 // rows of `bytes` bytes: the row stride of a chunk's padded rows, an odd multiple of 64
 __host__ __device__ constexpr int padded(int bytes) { return ((bytes + 63) & ~127) + 64; }
-__host__ __device__ constexpr int up128(int bytes) { return (bytes + 127) & ~127; }
 
 // chunk j of a CTA's share of a uniform batch, parts first, first + stride, ...
 __device__ __forceinline__ ChunkDesc uniform_chunk(const Uniform &u, int64_t first, int j, int stride)
@@ -329,30 +322,13 @@ __device__ __forceinline__ void copy_chunks(const RingParams &rp, uint8_t *smem,
         {
             const int l = __ffs(todo) - 1;
             j = j0 + l;
-            // The computing warps pass the chunks in order, so a chunk's
-            // barrier answers for the older ones too.  A wait on parity cannot
-            // tell a phase from the one two ahead: never further than kRecs
-            // past what is known.
-            const int dep = __shfl_sync(0xffffffffu, d.dep, l);
-            while (gone < dep && ok)
-            {
-                const int to = min(dep, gone + kRecs);
-                ok = __all_sync(0xffffffffu, tc::mbar_wait_bounded(&empty[to % kRecs], (to / kRecs) & 1, limit));
-                gone = to;
-            }
+            const int s = j % kRecs;
+            ok = wait_gone(empty, __shfl_sync(0xffffffffu, d.dep, l), gone, limit) &&
+                 wait_landed(full, empty, __shfl_sync(0xffffffffu, d.land, l), gone, limit);
             if (!ok)
             {
                 if (lane == 0)
                     ring_flag(1);
-                break;
-            }
-            const int s = j % kRecs, land = __shfl_sync(0xffffffffu, d.land, l);
-            if (land >= 0)
-                ok = __all_sync(0xffffffffu, tc::mbar_wait_bounded(&full[land % kRecs], (land / kRecs) & 1, limit));
-            if (!ok)
-            {
-                if (lane == 0)
-                    ring_flag(4);
                 break;
             }
             if (lane == l && l % kCopyWarps == cw)
@@ -510,26 +486,26 @@ __global__ void __launch_bounds__(kThreads, 1) f64_ring_kernel(const __grid_cons
 
 int launch_ring(const RingParams &rp, int ctas, cudaStream_t s)
 {
-    static std::once_flag once;
-    static cudaError_t attr;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute((const void *)&f64_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev >= 64)
+        return e != cudaSuccess ? cuda_fail(e, "cudaGetDevice") : KAMI_ERR_UNSUPPORTED;
+    static std::once_flag once[64];
+    static cudaError_t attr[64];
+    std::call_once(once[dev], [&] {
+        attr[dev] =
+            cudaFuncSetAttribute((const void *)&f64_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     });
-    if (attr != cudaSuccess)
-        return cuda_fail(attr, "cudaFuncSetAttribute(f64_ring_kernel)");
+    if (attr[dev] != cudaSuccess)
+        return cuda_fail(attr[dev], "cudaFuncSetAttribute(f64_ring_kernel)");
     void *args[] = {const_cast<RingParams *>(&rp)};
-    const cudaError_t e =
-        cudaLaunchKernel((const void *)&f64_ring_kernel, dim3(ctas), dim3(kThreads), args, kSmem, s);
+    e = cudaLaunchKernel((const void *)&f64_ring_kernel, dim3(ctas), dim3(kThreads), args, kSmem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(f64_ring_kernel)");
     return KAMI_OK;
 }
 
 } // namespace
-
-const void *grouped_f64s_fn() { return (const void *)&f64_ring_kernel; }
-
-int grouped_f64s_threads() { return kThreads; }
 
 int grouped_f64s_smem() { return kSmem; }
 
@@ -582,17 +558,12 @@ size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *
         problems += l.size();
     out->clear();
     out->reserve((problems + problems / 2) * sizeof(ChunkDesc));
-    struct Span
-    {
-        int from, to;
-    };
-    std::vector<Span> at_of; // ring bytes of the list's chunks
+    Placer placer(kRing);
     for (size_t c = 0; c < lists.size(); ++c)
     {
         (*begin)[c] = (int)count;
-        const size_t base = count;
-        at_of.clear();
-        int head = 0, deal = 0, gone = -1;
+        placer.clear();
+        int deal = 0;
         for (int i : lists[c])
         {
             int mb = 0, nb = 0;
@@ -614,24 +585,7 @@ size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *
                     d.r.inv = (65535u + (uint32_t)nf) / (uint32_t)nf;
                     for (int k0 = 0; k0 < k; k0 += kc)
                     {
-                        const int j = (int)(count - base), kv = std::min(kc, k - k0);
-                        const int at = head + bytes > kRing ? 0 : head, end = at + bytes;
-                        // The chunks whose bytes this one takes: the oldest that are
-                        // left, after those behind the place where the ring starts
-                        // again.  Never fewer than for the previous chunk, which may
-                        // have taken part of an older one's bytes, and this the rest.
-                        gone = std::max(gone, j - kRecs);
-                        int q = gone + 1;
-                        while (q < j && at < head && at_of[q].from >= head)
-                            ++q;
-                        for (; q < j && at_of[q].from < end && at < at_of[q].to; ++q)
-                            gone = q;
-                        d.dep = gone;
-                        head = end;
-                        at_of.push_back(Span{at, end});
-                        int fly = bytes;
-                        for (d.land = j - 1; d.land > gone && fly < kAhead; --d.land)
-                            fly += at_of[d.land].to - at_of[d.land].from;
+                        const int kv = std::min(kc, k - k0), at = placer.place(bytes, &d.dep, &d.land);
                         d.r.sa = (uint32_t)at;
                         d.r.sb = (uint32_t)(at + up128(m * pitch));
                         d.r.pitch_k = (uint32_t)(pitch | kv << 16);

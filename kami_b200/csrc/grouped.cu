@@ -462,12 +462,11 @@ using namespace kami;
 struct kami_grouped_plan
 {
     int in_type, out_type, count, ctas, smem;
-    int kernel = 0; // 0: mma.sync warp grids (grouped_kernel), 1: tcgen05 (grouped_tc05_kernel),
+    int kernel = 0; // 0: mma.sync warp grids (grouped_kernel), 1: tcgen05 (h16_ring_kernel),
                     // 2: FP64 ring (f64_ring_kernel)
     int tc_m64 = 0, tc_m128 = 0; // tcgen05 plans: problems on M = 64 / M = 128 MMAs
-    bool packed = false;         // tcgen05 plans: some work item holds several problems
     int small_begin = 0, small_end = 0; // desc range of single-warp problems
-    void *d_desc = nullptr; // GroupedDesc per problem; chunk descriptors for FP64 ring plans
+    void *d_desc = nullptr; // GroupedDesc per problem; the ring kernels' own descriptors
     int *d_begin = nullptr;
     int cfg_hist[kCfgs] = {0};
     int64_t flops = 0, bytes = 0;
@@ -552,7 +551,7 @@ static int launch_grouped(const kami_grouped_plan *plan, const void *A, const vo
     p.small_begin = plan->small_begin;
     p.small_end = plan->small_end;
     if (plan->kernel == 1)
-        return grouped_tc05_launch(p, plan->in_type == KAMI_BF16, plan->packed, plan->ctas, s);
+        return grouped_tc05_launch(p, plan->d_desc, plan->in_type == KAMI_BF16, plan->ctas, s);
     if (plan->kernel == 2)
         return grouped_f64s_launch(p, plan->d_desc, plan->ctas, s);
     void *args[] = {&p};
@@ -577,13 +576,13 @@ static int free_plan(kami_grouped_plan *pl)
 
 // Build descriptors + LPT schedule for `count` problems (host arrays) with
 // the given partitions and upload them.  kernel 1 (FP16 / BF16 only) is the
-// tcgen05 kernel, kernel 2 (FP64 only) the ring kernel: every problem
+// tcgen05 ring kernel, kernel 2 (FP64 only) the DMMA ring kernel: every problem
 // goes through their CTA pipelines (no single-warp problems); the tcgen05
 // kernel's cost model is its bytes plus a fixed per-problem latency.
 static int build_plan(int in_type, int out_type, int count, const int *M, const int *N, const int *K,
                       const int64_t *ao, const int64_t *bo, const int64_t *co, const int *cfg,
                       kami_grouped_plan **out, const int *lda = nullptr, const int *ldb = nullptr,
-                      const int *ldc = nullptr, int kernel = 0, bool pack = false)
+                      const int *ldc = nullptr, int kernel = 0)
 {
     int dev = 0, sms = 0, occ = 0;
     cudaError_t e;
@@ -592,26 +591,19 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return cuda_fail(e, "cudaDeviceGetAttribute");
     const bool tc = kernel == 1, staged = kernel == 2;
-    const void *fn = tc ? grouped_tc05_fn(in_type == KAMI_BF16, false) : staged ? grouped_f64s_fn() : grouped_fn(in_type);
     const int smem = tc ? grouped_tc05_smem() : staged ? grouped_f64s_smem() : grouped_smem(in_type);
-    const int threads = tc ? grouped_tc05_threads() : staged ? grouped_f64s_threads() : kThreads;
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
-        return cuda_fail(e, "cudaFuncSetAttribute(grouped kernel)");
-    if (tc && (e = cudaFuncSetAttribute(grouped_tc05_fn(in_type == KAMI_BF16, true),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
-        return cuda_fail(e, "cudaFuncSetAttribute(grouped kernel)");
-    // all of the SM's unified L1 / shared memory as shared memory, so the
-    // occupancy below counts every CTA that fits
-    for (int pk = 0; tc && pk < 2; ++pk)
-        if ((e = cudaFuncSetAttribute(grouped_tc05_fn(in_type == KAMI_BF16, pk == 1),
-                                      cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
-            return cuda_fail(e, "cudaFuncSetAttribute(grouped kernel carveout)");
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem)) != cudaSuccess)
-        return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (tc)
-        occ = grouped_tc05_ctas_per_sm(); // sized for two per SM; the query reports one
+    if (!tc && !staged) // (the ring kernels run one CTA per SM)
+    {
+        const void *fn = grouped_fn(in_type);
+        if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+            return cuda_fail(e, "cudaFuncSetAttribute(grouped kernel)");
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, smem)) != cudaSuccess)
+            return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+    }
     occ = std::max(occ, 1);
-    const int ctas = std::max(1, std::min(count, sms * occ));
+    // tcgen05 plans have several lists of problems per CTA
+    const int per_cta = tc ? grouped_tc05_lists() : 1;
+    const int ctas = std::max(1, std::min(count, sms * occ)), nlists = ctas * per_cta;
     const int esz = in_type == KAMI_F64 ? 8 : 2;
     const int osz = out_type == KAMI_F64 ? 8 : out_type == KAMI_F32 ? 4 : 2;
     // FLOP per byte where compute and HBM meet (the tcgen05 kernel's MMAs
@@ -638,92 +630,17 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
         if (!tc && !staged)
             pl->cfg_hist[cfg[i]]++;
     }
-    // Work items.  tcgen05 plans put several small problems in one item: their
-    // A rows stacked in the item's 128-row A tile, their B rows (each problem's
-    // rounded up to 16) in its 128-row B tile, so that one chain of MMAs computes
-    // every problem's C block on the accumulator's diagonal (the off-diagonal
-    // blocks are computed and never read) and the issuing thread, the loaders
-    // and the epilogue pay their fixed per-item costs once for all of them.
-    // pk[i]: row offset | column offset << 8 | problems in the item << 16.
-    std::vector<std::vector<int>> items;
-    std::vector<int> pk(count, 0);
-    if (tc && pack)
-    {
-        std::vector<int> small;
-        for (int i = 0; i < count; ++i)
-        {
-            if (M[i] <= 64 && ((N[i] + 15) & ~15) <= 64)
-                small.push_back(i);
-            else
-                items.push_back({i});
-        }
-        // similar K together (an item runs to its largest K), then tall first
-        std::stable_sort(small.begin(), small.end(), [&](int a, int b) {
-            return K[a] != K[b] ? K[a] > K[b] : M[a] > M[b];
-        });
-        struct Bin
-        {
-            int item, m, n, k0;
-        };
-        std::vector<Bin> open; // the most recent bins, first fit
-        for (int i : small)
-        {
-            const int n16 = (N[i] + 15) & ~15;
-            bool placed = false;
-            for (Bin &b : open)
-                if (b.m + M[i] <= 128 && b.n + n16 <= 128 && (int)items[b.item].size() < 4 && b.k0 - K[i] <= 32)
-                {
-                    pk[i] = b.m | (b.n << 8);
-                    items[b.item].push_back(i);
-                    b.m += M[i];
-                    b.n += n16;
-                    placed = true;
-                    break;
-                }
-            if (!placed)
-            {
-                items.push_back({i});
-                open.push_back(Bin{(int)items.size() - 1, M[i], n16, K[i]});
-                if (open.size() > 16)
-                    open.erase(open.begin());
-            }
-        }
-        for (const auto &it : items)
-        {
-            for (int i : it)
-                pk[i] |= (int)it.size() << 16;
-            pl->packed = pl->packed || it.size() > 1;
-        }
-    }
-    // members of item t: without packing, problem t alone
-    const bool packing = tc && pack;
-    const int nitems = packing ? (int)items.size() : count;
-    auto first_of = [&](int t) { return packing ? items[t].data() : &order[t]; };
-    auto size_of = [&](int t) { return packing ? (int)items[t].size() : 1; };
-    std::vector<double> icost(nitems, 2048.0);
-    std::vector<int> iorder(nitems);
-    for (int t = 0; t < nitems; ++t)
-    {
-        int mt = 0;
-        for (const int *i = first_of(t); i != first_of(t) + size_of(t); ++i)
-        {
-            icost[t] += cost[*i] - 2048.0;
-            mt += M[*i];
-        }
-        if (tc)
-            (mt <= 64 ? pl->tc_m64 : pl->tc_m128) += size_of(t);
-        iorder[t] = t;
-    }
-    std::stable_sort(iorder.begin(), iorder.end(), [&](int a, int b) { return icost[a] > icost[b]; });
+    if (tc)
+        pl->tc_m128 = count; // (every problem on M = 128 MMAs, h16_ring.cu)
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     typedef std::pair<double, int> Load;
     std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
-    for (int c = 0; c < ctas; ++c)
+    for (int c = 0; c < nlists; ++c)
         heap.push(Load(0.0, c));
-    std::vector<std::vector<int>> lists(ctas); // work items per CTA
+    std::vector<std::vector<int>> lists(nlists);
     std::vector<int> smalls;
-    for (int t : iorder)
+    for (int i : order)
     {
-        const int i = *first_of(t);
         if (cfg[i] == 7 && kernel == 0)
         {
             smalls.push_back(i); // longest first, spread over all warps round-robin
@@ -731,57 +648,41 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
         }
         Load l = heap.top();
         heap.pop();
-        lists[l.second].push_back(t);
-        heap.push(Load(l.first + icost[t], l.second));
+        lists[l.second].push_back(i);
+        heap.push(Load(l.first + cost[i], l.second));
     }
     std::vector<GroupedDesc> desc;
     desc.reserve(count);
     std::vector<int> begin(ctas + 1, 0);
-    for (int c = 0; c < ctas && !staged; ++c)
+    for (int c = 0; c < ctas && kernel == 0; ++c)
     {
         begin[c] = (int)desc.size();
-        for (int t : lists[c])
-        {
-            // tcgen05 plans: the item's extent in every member (see item_at in
-            // grouped_tc05.cu): count | Mt << 3 | (Nt / 16) << 11 | Kt << 15
-            int mt = 0, nt = 0, kt = 0;
-            const int *members = first_of(t), *members_end = members + size_of(t);
-            for (const int *m = members; m != members_end; ++m)
-            {
-                const int i = *m;
-                mt = std::max(mt, (pk[i] & 0xff) + M[i]);
-                nt = std::max(nt, ((pk[i] >> 8) & 0xff) + ((N[i] + 15) & ~15));
-                kt = std::max(kt, K[i]);
-            }
-            const int ext = tc ? size_of(t) | (mt << 3) | ((nt / 16) << 11) | (kt << 15) : 0;
-            for (const int *m = members; m != members_end; ++m)
-            {
-                const int i = *m;
-                desc.push_back(GroupedDesc{M[i], N[i], K[i], tc ? pk[i] : cfg[i], ao[i], bo[i], co[i],
-                                           lda ? lda[i] : K[i], ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i], ext});
-            }
-        }
+        for (int i : lists[c])
+            desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], lda ? lda[i] : K[i],
+                                       ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i]});
     }
     begin[ctas] = (int)desc.size();
     pl->small_begin = (int)desc.size();
     for (int i : smalls)
         desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], lda ? lda[i] : K[i],
-                                   ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i], 0});
+                                   ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i]});
     pl->small_end = (int)desc.size();
-    // FP64 ring plans: the chunks of every CTA's problems instead of the problems
+    // ring plans: the kernels' own descriptors instead
     std::vector<char> chunks;
     if (staged)
         f64_ring_schedule(lists, M, N, K, ao, bo, co, &chunks, &begin);
-    const void *src = staged ? (const void *)chunks.data() : (const void *)desc.data();
-    const size_t src_bytes = staged ? chunks.size() : sizeof(GroupedDesc) * desc.size();
+    else if (tc)
+        h16_ring_schedule(lists, M, N, K, ao, bo, co, lda, ldb, ldc, &chunks, &begin);
+    const void *src = kernel ? (const void *)chunks.data() : (const void *)desc.data();
+    const size_t src_bytes = kernel ? chunks.size() : sizeof(GroupedDesc) * desc.size();
     if ((e = cudaMalloc(&pl->d_desc, std::max(src_bytes, (size_t)16))) != cudaSuccess ||
-        (e = cudaMalloc(&pl->d_begin, sizeof(int) * (ctas + 1))) != cudaSuccess)
+        (e = cudaMalloc(&pl->d_begin, sizeof(int) * begin.size())) != cudaSuccess)
     {
         free_plan(pl);
         return cuda_fail(e, "cudaMalloc(grouped plan)");
     }
     if ((e = cudaMemcpy(pl->d_desc, src, src_bytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(pl->d_begin, begin.data(), sizeof(int) * (ctas + 1), cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = cudaMemcpy(pl->d_begin, begin.data(), sizeof(int) * begin.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
     {
         free_plan(pl);
         return cuda_fail(e, "cudaMemcpy(grouped plan)");
@@ -920,7 +821,7 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
     if (count < 0 || (count > 0 && (!M || !N || !K || !a_offsets || !b_offsets || !c_offsets)))
         return fail(KAMI_ERR_INVALID_VALUE, "grouped: bad count or null shape/offset arrays");
     const bool force_mma = (flags & KAMI_PLAN_MMA_SYNC) != 0, force_tc = (flags & KAMI_PLAN_TCGEN05) != 0,
-               force_st = (flags & KAMI_PLAN_STAGED) != 0, pack = (flags & KAMI_PLAN_PACK) != 0;
+               force_st = (flags & KAMI_PLAN_STAGED) != 0;
     if ((int)force_mma + (int)force_tc + (int)force_st > 1)
         return fail(KAMI_ERR_INVALID_VALUE,
                     "grouped: KAMI_PLAN_MMA_SYNC, KAMI_PLAN_TCGEN05 and KAMI_PLAN_STAGED are exclusive");
@@ -1040,14 +941,14 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
         return build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), plan);
     if (force_tc || force_st || !tune || count == 0)
         return build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), plan,
-                          nullptr, nullptr, nullptr, alt, pack);
+                          nullptr, nullptr, nullptr, alt);
     // autotuned, kernel not forced: build both kernels' plans, time each on
     // scratch buffers of the plan's extent, keep the faster
     kami_grouped_plan *pl[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; ++k)
     {
         int st = build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), &pl[k],
-                            nullptr, nullptr, nullptr, k == 0 ? 0 : alt, pack);
+                            nullptr, nullptr, nullptr, k == 0 ? 0 : alt);
         if (st)
         {
             free_plan(pl[0]);
@@ -1343,7 +1244,7 @@ extern "C" int kami_gemm_grouped_noalloc(kami_dtype_t in_type, kami_dtype_t out_
             const int i = g_na_order[r];
             const int slot = g_na_cta[i] < 0 ? small_slot++ : g_na_heap[g_na_cta[i]]++;
             g_na_desc[slot] = GroupedDesc{M[i], N[i], K[i], cfg_heuristic(in_type, M[i], N[i], K[i]),
-                                          a_offsets[i], b_offsets[i], c_offsets[i], K[i], K[i], N[i], 0};
+                                          a_offsets[i], b_offsets[i], c_offsets[i], K[i], K[i], N[i]};
         }
     }
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

@@ -1,7 +1,7 @@
 // grouped.cuh -- device descriptors of the uneven (grouped) batched GEMM,
 // shared by its three kernels: the mma.sync warp-grid kernel (grouped.cu),
-// the tcgen05 kernel (grouped_tc05.cu, FP16 / BF16) and the FP64 ring
-// kernel (f64_ring.cu).
+// the tcgen05 ring kernel (h16_ring.cu, FP16 / BF16) and the FP64 ring kernel
+// (f64_ring.cu).
 #pragma once
 #include <vector>
 
@@ -16,7 +16,6 @@ struct GroupedDesc
     int M, N, K, cfg;
     int64_t a_off, b_off, c_off;
     int lda, ldb, ldc;
-    int ext; // tcgen05 plans: extent of the work item this problem belongs to (grouped_tc05.cu, item_at)
 };
 
 struct GroupedParams
@@ -32,23 +31,23 @@ struct GroupedParams
     int small_begin, small_end; // desc range of problems run by single warps
 };
 
-// tcgen05 grouped kernel (grouped_tc05.cu): entry point, launch geometry and
-// the device status of its bounded waits.
-const void *grouped_tc05_fn(bool bf16, bool packed);
-int grouped_tc05_threads();
+// 16-bit ring kernel (h16_ring.cu): plans, and uniform batches
+// (h16_ring_launch)
 int grouped_tc05_smem();
-int grouped_tc05_ctas_per_sm();
-int grouped_tc05_launch(const GroupedParams &p, bool bf16, bool packed, int ctas, cudaStream_t s);
+int grouped_tc05_lists(); // problem lists of a CTA
+void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
+                       const int64_t *ao, const int64_t *bo, const int64_t *co, const int *lda, const int *ldb,
+                       const int *ldc, std::vector<char> *out, std::vector<int> *begin);
+int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, cudaStream_t s);
+int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s);
 int grouped_tc05_read_error(int *flag);
 
 // FP64 ring kernel (f64_ring.cu): plans, and uniform batches (f64_ring_launch)
-const void *grouped_f64s_fn();
-int grouped_f64s_threads();
 int grouped_f64s_smem();
-int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s);
 size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
                          const int64_t *ao, const int64_t *bo, const int64_t *co, std::vector<char> *out,
                          std::vector<int> *begin);
+int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s);
 int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
 int f64_ring_read_error(int *flag);
 

@@ -21,6 +21,7 @@ int spgemm_tc05_read_error(int *flag);
 int split_read_error(int *flag);
 int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream);
 int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
+int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s);
 
 static thread_local char g_err[512] = "no error";
 
@@ -431,6 +432,36 @@ int gemm_batched_hinted(kami_dtype_t in_type, kami_dtype_t out_type, kami_partit
     g.num_iter = num_iter;
     g.one_per_sm = one_per_sm;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+
+    // Streamed 16-bit problems: the ring kernel, when the choice is left to the
+    // library, where the other kernels mostly pad (us below: FP16 in, FP32 out).
+    // The per-problem mma.sync kernel (M <= 32 or N < 32) keeps compiled sizes
+    // up to 16^3 (300 MB 60 against 160), and below 16 MB what fits 32^3 (4 MB of
+    // 32^3 3.2 against 4.6; 40 MB 25 against 14) and N that is not a multiple
+    // of 8, whose rows the ring stores in pieces (4 MB of 24 x 100 x 72 7.3
+    // against 12.6; 40 MB 70 against 34); elsewhere the ring is ahead, up to 11x
+    // (300 MB of 100 x 16 x 40 635 against 58, of 20 x 20 x 128 1073 against 94).
+    // The TMA kernels keep M > 64 (300 MB of 72 x 88 x 104 64 against 68, 128^3 54
+    // against 61), 64 rows of 64 columns or more (64^3 55 against 55 to 64),
+    // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
+    // 12.0 against 13.6) and N that is not a multiple of 8 (300 MB of
+    // 50 x 33 x 64 117 against 140); other blocks of up to 64 rows take the ring
+    // (48^3 84 against 55, 40^3 119 against 55, 64 x 40 x 64 67 against 55,
+    // 33 x 128 x 40 88 against 63).
+    if (in_type != KAMI_F64 && variant == KAMI_VARIANT_AUTO && partition == KAMI_PARTITION_AUTO && P == 0 &&
+        alloc_warps == 0 && num_iter <= 4 && M <= 128 && N <= 128 && K <= 128 && K % 8 == 0 &&
+        a_layout == KAMI_A_ROW_MK && b_layout == KAMI_B_REF_NK && !(reinterpret_cast<uintptr_t>(A) & 15) &&
+        !(reinterpret_cast<uintptr_t>(B) & 15) && lda % 8 == 0 && ldb % 8 == 0 &&
+        (batch == 1 || (strideA % 8 == 0 && strideB % 8 == 0)) && lda <= 0x3fffffff && ldb <= 0x3fffffff &&
+        ldc <= 0x7fffffff)
+    {
+        const int largest = std::max(M, std::max(N, K));
+        const double bytes = (double)batch * ((double)(M + N) * K * esz + (double)M * N * osz);
+        const bool tma = tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout);
+        if (tma ? N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256
+                : largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0)))
+            return h16_ring_launch(g, in_type, s);
+    }
 
     if (variant == KAMI_VARIANT_TCGEN05 || variant == KAMI_VARIANT_TCGEN05_TS ||
         (variant == KAMI_VARIANT_AUTO && tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout)))
