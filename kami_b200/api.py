@@ -10,6 +10,7 @@ NUM_ALLOC_RANK_BLOCK and ``num_iter`` is NUM_ITER.
 from __future__ import annotations
 
 import ctypes
+import os
 
 import torch
 
@@ -24,6 +25,7 @@ _AL = {"row_mk": _lib.A_ROW_MK, "col_mk": _lib.A_COL_MK}
 _BL = {"ref_nk": _lib.B_REF_NK, "row_kn": _lib.B_ROW_KN}
 
 
+_OPS_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libkami_torch_ops.so")
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _cur_device = getattr(torch._C, "_cuda_getDevice", None)
 
@@ -84,6 +86,34 @@ def _on(*tensors) -> _OnDevice:
     return _OnDevice(_device_index(*tensors))
 
 
+_calls = None
+
+
+def _native():
+    """The C++ forms of gemm_batched, spmm and spgemm (module kami_calls of
+    libkami_torch_ops.so, kami_b200/torch_ops/kami_calls.cpp), or False where
+    that library is not built.  They return NotImplemented for what they leave
+    to the code here, and a status for a call that failed."""
+    global _calls
+    if _calls is None:
+        L = load()
+        calls = False
+        if os.path.exists(_OPS_PATH):
+            import importlib.machinery
+            import importlib.util
+            loader = importlib.machinery.ExtensionFileLoader("kami_calls", _OPS_PATH)
+            try:
+                calls = importlib.util.module_from_spec(
+                    importlib.util.spec_from_file_location("kami_calls", _OPS_PATH, loader=loader))
+                calls.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
+                    L.kami_gemm_batched, L.kami_spmm_bsr, L.kami_spgemm_bsr_symbolic, L.kami_spgemm_bsr_fill_colidx,
+                    L.kami_spgemm_bsr_numeric_variant)))
+            except ImportError:  # built for another torch
+                calls = False
+        _calls = calls
+    return _calls
+
+
 def _as3(x: torch.Tensor) -> torch.Tensor:
     return x.unsqueeze(0) if x.dim() == 2 else x
 
@@ -114,6 +144,13 @@ def gemm_batched(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None = None
     B: [batch, N, K] (ref_nk) or [batch, K, N] (row_kn).
     Returns C [batch, M, N]: float32 for 16-bit inputs unless ``out_dtype``
     (float16 / bfloat16) is given, float64 for float64 inputs."""
+    if stream is None and (calls := _calls if _calls is not None else _native()):
+        r = calls.gemm_batched(A, B, C, out_dtype, _AL.get(a_layout), _BL.get(b_layout), _PART.get(partition),
+                               _VAR.get(variant), P, alloc_warps, num_iter, alpha, beta)
+        if r is not NotImplemented:
+            if type(r) is int:
+                check(r)
+            return r
     squeeze = A.dim() == 2
     A3, B3 = _as3(A), _as3(B)
     if A3.dtype != B3.dtype:
@@ -475,6 +512,13 @@ def spgemm_numeric_bound(A: BSR, B: BSR, row_ptr_c, col_idx_c, C_values, *, alph
 
 def spgemm(A: BSR, B: BSR, out_dtype=torch.float32, *, num_iter=1, variant: str = "auto", stream=None) -> BSR:
     """C = A * B: symbolic, column fill, numeric (the reference's sequence)."""
+    if stream is None and A.block_cols == B.block_rows and (calls := _calls if _calls is not None else _native()):
+        r = calls.spgemm(A.row_ptr, A.col_idx, A.values, A.block_rows, A.block_cols, B.row_ptr, B.col_idx, B.values,
+                         B.block_cols, out_dtype, num_iter, _VAR.get(variant))
+        if r is not NotImplemented:
+            if type(r) is int:
+                check(r)
+            return BSR(*r, B.block_cols)
     rpc, nnz = spgemm_symbolic(A, B, stream)
     cic = spgemm_fill_colidx(A, B, rpc, nnz, stream)
     vals = spgemm_numeric(A, B, rpc, cic, out_dtype, num_iter=num_iter, variant=variant, stream=stream)
@@ -514,6 +558,13 @@ def spmm(A: BSR, B: torch.Tensor, C: torch.Tensor | None = None, *, b_layout: st
     """Block SpMM (kami_spmm_bsr): C [16 mb, N] = A * B for a BSR matrix A and
     a dense B, [K, N] (row_kn, torch's A @ B) or [N, K] (ref_nk, the
     reference's layout: C = A * B^T).  FP16/BF16 operands, FP32 accumulation."""
+    if stream is None and (calls := _calls if _calls is not None else _native()):
+        r = calls.spmm(A.row_ptr, A.col_idx, A.values, A.block_rows, A.block_cols, B, C, out_dtype, _BL.get(b_layout),
+                       num_iter, alpha, beta)
+        if r is not NotImplemented:
+            if type(r) is int:
+                check(r)
+            return r
     K = A.block_cols * 16
     if B.dim() != 2:
         raise ValueError("B must be 2-D")

@@ -72,16 +72,19 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
     return LIB
 
 
-OPS_SRC = os.path.join(HERE, "torch_ops", "kami_torch_ops.cpp")
+OPS_SRCS = [os.path.join(HERE, "torch_ops", f) for f in ("kami_torch_ops.cpp", "kami_calls.cpp")]
 OPS_LIB = os.path.join(HERE, "libkami_torch_ops.so")
 
 
 def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
-    """torch.ops.kami (the differentiable batched GEMM as a C++ torch operator,
-    kami_b200/torch_ops/) linked against libkami_b200.so and libtorch."""
+    """torch.ops.kami (the differentiable batched GEMM as a C++ torch operator)
+    and the module kami_calls (api calls without ctypes), kami_b200/torch_ops/,
+    in one library linked against libkami_b200.so and libtorch."""
+    import sysconfig
+
     import torch
     tdir = os.path.dirname(torch.__file__)
-    srcs = [OPS_SRC, os.path.join(INCLUDE, "kami.h")]
+    srcs = [*OPS_SRCS, os.path.join(INCLUDE, "kami.h")]
     if not force and os.path.exists(OPS_LIB) and os.path.getmtime(OPS_LIB) >= max(os.path.getmtime(x) for x in srcs) \
             and os.path.getmtime(OPS_LIB) >= os.path.getmtime(LIB):
         return OPS_LIB
@@ -90,8 +93,9 @@ def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
     tmp = OPS_LIB + ".tmp"
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
            "-I", os.path.join(tdir, "include"), "-I", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
-           "-I", os.path.join(cuda_home, "include"), "-I", INCLUDE, OPS_SRC, "-o", tmp,
-           "-L", os.path.join(tdir, "lib"), "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           "-I", os.path.join(cuda_home, "include"), "-I", INCLUDE,
+           "-I", sysconfig.get_paths()["include"], *OPS_SRCS, "-o", tmp,
+           "-L", os.path.join(tdir, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
            "-L", HERE, "-l:libkami_b200.so", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + os.path.join(tdir, "lib")]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
