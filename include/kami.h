@@ -449,6 +449,16 @@ int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type
                                     const int *row_ptr_c, const int *col_idx_c, void *val_c,
                                     int64_t nnz_c, double alpha, double beta, int num_iter, void *stream);
 
+/* kami_spgemm_bsr_fill_colidx and kami_spgemm_bsr_numeric_variant in one call:
+ * col_idx_c is written as well (row_ptr_c from kami_spgemm_bsr_symbolic, nnz_c
+ * its last entry).  One launch where the block-row kernel runs and nb <= 16384. */
+int kami_spgemm_bsr_fill_numeric(kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr,
+                                 int mb, int kb, int nb,
+                                 const int *row_ptr_a, const int *col_idx_a, const void *val_a,
+                                 const int *row_ptr_b, const int *col_idx_b, const void *val_b,
+                                 const int *row_ptr_c, int *col_idx_c, void *val_c,
+                                 int64_t nnz_c, double alpha, double beta, int num_iter, void *stream);
+
 /* ------------------------------------------------------------------------ */
 /* Block SpMM: BSR (16 x 16 tiles) times dense                              */
 /* ------------------------------------------------------------------------ */

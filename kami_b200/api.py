@@ -106,8 +106,7 @@ def _native():
                 calls = importlib.util.module_from_spec(
                     importlib.util.spec_from_file_location("kami_calls", _OPS_PATH, loader=loader))
                 calls.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
-                    L.kami_gemm_batched, L.kami_spmm_bsr, L.kami_spgemm_bsr_symbolic, L.kami_spgemm_bsr_fill_colidx,
-                    L.kami_spgemm_bsr_numeric_variant)))
+                    L.kami_gemm_batched, L.kami_spmm_bsr, L.kami_spgemm_bsr_symbolic, L.kami_spgemm_bsr_fill_numeric)))
             except ImportError:  # built for another torch
                 calls = False
         _calls = calls

@@ -581,6 +581,7 @@ struct SpNumArgs
 {
     int mb, nb;
     const int *rpa, *cia, *rpb, *cib, *rpc, *cic;
+    int *cic_out; // the array of cic, where the pass fills it
     const uint16_t *va, *vb;
     void *vc;
     int64_t nnzc;
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(256) spgemm_numeric_kernel(const SpNumArgs p)
 }
 
 // ---------------------------------------------------------------------------
-// numeric, one CTA per block-row of C (16-byte aligned tiles)
+// numeric, rows beyond the capacities of the kernel below (16-byte aligned tiles)
 //
 // The C tiles of block-row i all multiply the same A tiles A(i, k) and search
 // the same B block-rows k for their column j.  So the CTA stages, once, the
@@ -693,14 +694,12 @@ __global__ void __launch_bounds__(256) spgemm_numeric_kernel(const SpNumArgs p)
 // ascending k, as the reference's sparse accumulator does.  Rows whose A
 // tiles or B lists exceed the staging capacity read them from global memory.
 // ---------------------------------------------------------------------------
-constexpr int kRowWarps = 8;
-constexpr int kMaxATiles = 32;   // 16 KB of A tiles (about 28 KB per CTA: 8 CTAs per SM)
 constexpr int kMaxBList = 2048;  // 8 KB of B column indices
 
 // The row's C tiles pulled one at a time (the per-tile search form); the
-// CTA's shared buffers are passed in: sA kMaxATiles * 512 bytes, sB
-// kRowWarps * 512, sList kMaxBList ints, sOff kMaxATiles + 1, sK kMaxATiles.
-template <bool BF16, int WARPS, int MAXA = kMaxATiles>
+// CTA's shared buffers are passed in: sA MAXA * 512 bytes, sB WARPS * 512,
+// sList kMaxBList ints, sOff MAXA + 1, sK MAXA.
+template <bool BF16, int WARPS, int MAXA>
 __device__ __forceinline__ void numeric_row_pull(const SpNumArgs &p, const int i, uint8_t *sA, uint8_t *sB,
                                                  int *sList, int *sOff, int *sK)
 {
@@ -845,17 +844,6 @@ __device__ __forceinline__ void numeric_row_pull(const SpNumArgs &p, const int i
     }
 }
 
-template <bool BF16>
-__global__ void __launch_bounds__(kRowWarps * 32) spgemm_numeric_row_kernel(const SpNumArgs p)
-{
-    __shared__ __align__(16) uint8_t sA[kMaxATiles * 512];
-    __shared__ __align__(16) uint8_t sB[kRowWarps * 512]; // one B tile slot per warp
-    __shared__ int sList[kMaxBList];
-    __shared__ int sOff[kMaxATiles + 1];
-    __shared__ int sK[kMaxATiles];
-    numeric_row_pull<BF16, kRowWarps>(p, blockIdx.x, sA, sB, sList, sOff, sK);
-}
-
 // ---------------------------------------------------------------------------
 // numeric, one CTA per block-row of C, products pushed to their tiles
 //
@@ -863,27 +851,128 @@ __global__ void __launch_bounds__(kRowWarps * 32) spgemm_numeric_row_kernel(cons
 // pair -- about ten per tile at 1 % density -- in dependent shared-memory
 // loads, and each tile's B tile load is exposed.  Here the row's products
 // are enumerated once: all threads walk the flattened (A entry, B entry)
-// space, find each product's C position by one binary search in the row's
-// ColIdxC (staged in shared memory), and a counting sort by position
+// space, find each product's C position, and a counting sort by position
 // groups them per C tile (each tile's short list then re-sorted by
 // enumeration index, so products still accumulate in ascending k).  The
-// warps then take the tiles in turn; each streams its products' B tiles
-// with 16-byte cp.async into a two-slot ring (the next product's tile in
-// flight while the current one is multiplied), A tiles read from the staged
-// row.  Rows beyond the staging capacities fall back to the per-tile form.
+// position comes from a bitmap of the row's columns (words of 32 with their
+// running counts) when the kernel writes ColIdxC as well (FILL: the pass that
+// would only fill it takes 7 us more at n = 16384, 1 %), else from a binary
+// search in the row's ColIdxC.
+// The warps then take the tiles in turn.  A product's B tile goes straight from
+// global memory into the fragments of two m16n8k16 MMAs, kPushDepth products
+// ahead: a lane's columns are 2 gq and 2 gq + 1, so four 4-byte loads and four
+// byte permutes make both fragments, and C leaves as float4 (through a ring
+// in shared memory and ldmatrix, the stores' halves exchanged by shuffles:
+// n = 16384, 1 % 37.3 us against 34.5; 4096 rows of 6 tiles 51 against 48).
+// What bounds it is the longest rows: the mean CTA runs 32 thousand cycles (9 of
+// them before its first product), the longest 50 thousand.  Runs of C tiles
+// dealt to warps across rows were even, and slower: 42 .. 56 us, each run
+// searching its products anew.  Rows beyond the staging capacities fall back to
+// the per-tile form.
 // ---------------------------------------------------------------------------
-constexpr int kPushWarps = 4;     // 4-warp CTAs, ~31 KB each: seven per SM, every row of a 1024-row matrix in one wave
+// Warps of a CTA: eight while every block-row has a place at once (four CTAs of
+// eight warps per SM), so that a row takes less time (numeric pass of 300 rows
+// of 9 entries 13.9 us against 17.1, 128 rows 13.0 against 17.1); four past that
+// (4096 rows of 6 48 us against 63, 1024 rows of 10 34.4 against 35.1).
+constexpr int kPushWarps = 4, kPushWarpsFew = 8, kPushFewPerSm = 4;
 constexpr int kPushMaxC = 512;    // C tiles of a row
 constexpr int kPushMaxProd = 512; // products of a row
 constexpr int kPushMaxA = 24;     // A tiles of a row staged (12 KB)
-constexpr int kPushDepth = 4;     // B tiles in flight per warp
+constexpr int kPushDepth = 4;     // B tiles on their way per warp, in registers
+constexpr int kFillWords = 512;   // FILL: words of 32 block columns
 
-template <bool BF16>
-__global__ void __launch_bounds__(kPushWarps * 32) spgemm_numeric_push_kernel(const SpNumArgs p)
+// C tile c with alpha / beta in any output type: lane (gq, tq) holds columns
+// 4 tq .. 4 tq + 3 of rows gq (lo) and gq + 8 (hi).  beta == 0 never reads C.
+__device__ __noinline__ void push_store(const SpNumArgs &p, int64_t c, int gq, int tq, const float4 lo, const float4 hi)
 {
-    constexpr int kRowWarps = kPushWarps;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        const float4 v = h ? hi : lo;
+        const int at = (gq + 8 * h) * 16 + 4 * tq;
+        if (p.out_type == KAMI_F32)
+        {
+            float2 *o = reinterpret_cast<float2 *>(reinterpret_cast<float *>(p.vc) + c * 256 + at);
+            float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
+            if (p.alpha != 1.f || p.beta != 0.f)
+            {
+                float2 q = make_float2(0.f, 0.f), r = q;
+                if (p.beta != 0.f)
+                    q = o[0], r = o[1];
+                x = make_float2(p.alpha * x.x + p.beta * q.x, p.alpha * x.y + p.beta * q.y);
+                y = make_float2(p.alpha * y.x + p.beta * r.x, p.alpha * y.y + p.beta * r.y);
+            }
+            o[0] = x;
+            o[1] = y;
+        }
+        else
+        {
+            uint2 *o = reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.vc) + c * 256 + at);
+            const bool bf = p.out_type == KAMI_BF16;
+            const uint2 old = p.beta != 0.f ? *o : make_uint2(0u, 0u);
+            auto cvt = [&](float f, uint32_t was) -> uint32_t {
+                float y = p.alpha * f;
+                if (p.beta != 0.f)
+                    y += p.beta * to_float((uint16_t)was, bf);
+                return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
+            };
+            *o = make_uint2(cvt(v.x, old.x & 0xffff) | (cvt(v.y, old.x >> 16) << 16),
+                            cvt(v.z, old.y & 0xffff) | (cvt(v.w, old.y >> 16) << 16));
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t pack16(float x, float y, bool bf)
+{
+    if (bf)
+    {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        return *reinterpret_cast<const uint32_t *>(&v);
+    }
+    const __half2 v = __floats2half2_rn(x, y);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+// The row's columns from its bitmap: pre[w] = columns before word w, and
+// ColIdxC's entries.  By the whole CTA.
+__device__ __forceinline__ void row_columns(const uint32_t *bm, int words, int *pre, int *cic)
+{
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32)
+    {
+        int carry = 0;
+        for (int b = 0; b < words; b += 32)
+        {
+            const int v = b + lane < words ? __popc(bm[b + lane]) : 0;
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o)
+                    x += y;
+            }
+            if (b + lane < words)
+                pre[b + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < words; w += blockDim.x)
+    {
+        int at = pre[w];
+        for (uint32_t bits = bm[w]; bits; bits &= bits - 1)
+            cic[at++] = w * 32 + __ffs(bits) - 1;
+    }
+}
+
+template <bool BF16, bool FILL, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const __grid_constant__ SpNumArgs p)
+{
     __shared__ __align__(16) uint8_t sA[kPushMaxA * 512];
-    __shared__ __align__(16) uint8_t sB[kRowWarps * kPushDepth * 512]; // B slots per warp
+    __shared__ __align__(16) uint8_t sB[WARPS * 512]; // of the per-tile fallback
+    __shared__ uint32_t sBits[FILL ? kFillWords : 1];      // the row's columns
+    __shared__ int sPre[FILL ? kFillWords : 1];
     // one pool of indices (the per-tile fallback uses its first kMaxBList
     // entries as its list buffer): the row's ColIdxC, then per tile the
     // product count / range end; per product (A entry << 16) | C position
@@ -897,56 +986,74 @@ __global__ void __launch_bounds__(kPushWarps * 32) spgemm_numeric_push_kernel(co
     __shared__ int sRb[kPushMaxA];
     const int i = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int kT = kRowWarps * 32;
+    constexpr int kT = WARPS * 32;
     const int c0 = p.rpc[i];
     const int c1 = (int)min((int64_t)p.rpc[i + 1], p.nnzc); // tiles past the caller's bound are untouched
     if (c1 <= c0)
         return;
     const int nt = c1 - c0;
     const int a0 = p.rpa[i], na = p.rpa[i + 1] - a0;
-    if (nt > kPushMaxC || na > kPushMaxA)
+    const int words = (p.nb + 31) >> 5;
+    if constexpr (FILL)
+        for (int w = tid; w < words; w += kT)
+            sBits[w] = 0u;
+    bool pull = nt > kPushMaxC || na > kPushMaxA;
+    int np = 0;
+    if (!pull)
     {
-        numeric_row_pull<BF16, kPushWarps, kPushMaxA>(p, i, sA, sB, sPool, sOff, sK);
-        return;
-    }
-    // ---- stage: ColIdxC, B row ranges and their prefix, A tiles ----
-    for (int t = tid; t < nt; t += kT)
-    {
-        sCol[t] = p.cic[c0 + t];
-        sCnt[t] = 0;
-    }
-    if (warp == 0)
-    {
-        int len = 0;
-        if (lane < na)
+        // ---- stage: ColIdxC, B row ranges and their prefix, A tiles ----
+        for (int t = tid; t < nt; t += kT)
         {
-            const int k = p.cia[a0 + lane];
-            const int rb = p.rpb[k];
-            len = p.rpb[k + 1] - rb;
-            sK[lane] = k;
-            sRb[lane] = rb;
+            if constexpr (!FILL)
+                sCol[t] = p.cic[c0 + t];
+            sCnt[t] = 0;
         }
-        int pre = len;
+        if (warp == 0)
+        {
+            int len = 0;
+            if (lane < na)
+            {
+                const int k = p.cia[a0 + lane];
+                const int rb = p.rpb[k];
+                len = p.rpb[k + 1] - rb;
+                sK[lane] = k;
+                sRb[lane] = rb;
+            }
+            int pre = len;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int y = __shfl_up_sync(0xffffffffu, pre, o);
-            if (lane >= o)
-                pre += y;
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int y = __shfl_up_sync(0xffffffffu, pre, o);
+                if (lane >= o)
+                    pre += y;
+            }
+            if (lane < na)
+                sOff[lane] = pre - len;
+            if (lane == 31)
+                sOff[na] = pre;
         }
-        if (lane < na)
-            sOff[lane] = pre - len;
-        if (lane == 31)
-            sOff[na] = pre;
+        for (int e = warp; e < na; e += WARPS)
+            stage_tile(sA + e * 512, p.va + (int64_t)(a0 + e) * 256, lane);
+        __syncthreads();
+        np = sOff[na];
+        pull = np > kPushMaxProd;
     }
-    for (int e = warp; e < na; e += kRowWarps)
-        stage_tile(sA + e * 512, p.va + (int64_t)(a0 + e) * 256, lane);
-    __syncthreads();
-    const int np = sOff[na];
-    if (np > kPushMaxProd)
+    if (pull)
     {
         __syncthreads();
-        numeric_row_pull<BF16, kPushWarps, kPushMaxA>(p, i, sA, sB, sPool, sOff, sK);
+        if constexpr (FILL)
+        {
+            for (int e = a0 + tid; e < a0 + na; e += kT)
+            {
+                const int k = p.cia[e], b1 = p.rpb[k + 1];
+                for (int b = p.rpb[k]; b < b1; ++b)
+                    atomicOr(&sBits[p.cib[b] >> 5], 1u << (p.cib[b] & 31));
+            }
+            __syncthreads();
+            row_columns(sBits, words, sPre, p.cic_out + c0);
+            __syncthreads();
+        }
+        numeric_row_pull<BF16, WARPS, kPushMaxA>(p, i, sA, sB, sPool, sOff, sK);
         return;
     }
     // ---- enumerate the products and count them per C tile ----
@@ -964,6 +1071,14 @@ __global__ void __launch_bounds__(kPushWarps * 32) spgemm_numeric_push_kernel(co
         const int e = lo;
         const int eb = sRb[e] + (f - sOff[e]);
         const int j = p.cib[eb];
+        sPb[f] = eb;
+        if constexpr (FILL)
+        {
+            sPep[f] = e << 16;
+            sOrd[f] = j;
+            atomicOr(&sBits[j >> 5], 1u << (j & 31));
+            continue;
+        }
         int l = 0, h = nt;
         while (l < h)
         {
@@ -975,11 +1090,21 @@ __global__ void __launch_bounds__(kPushWarps * 32) spgemm_numeric_push_kernel(co
         }
         const bool hit = l < nt && sCol[l] == j;
         sPep[f] = hit ? ((e << 16) | l) : -1;
-        sPb[f] = eb;
         if (hit)
             atomicAdd(&sCnt[l], 1);
     }
     __syncthreads();
+    if constexpr (FILL)
+    {
+        row_columns(sBits, words, sPre, p.cic_out + c0);
+        for (int f = tid; f < np; f += kT)
+        {
+            const int j = sOrd[f], l = sPre[j >> 5] + __popc(sBits[j >> 5] & ((1u << (j & 31)) - 1));
+            sPep[f] |= l;
+            atomicAdd(&sCnt[l], 1);
+        }
+        __syncthreads();
+    }
     // ---- exclusive scan of the counts (warp 0, 32 consecutive entries per lane) ----
     if (warp == 0)
     {
@@ -1032,98 +1157,111 @@ __global__ void __launch_bounds__(kPushWarps * 32) spgemm_numeric_push_kernel(co
     __syncthreads();
 
     // ---- multiply: warp w takes the contiguous tile range [t0, t1), whose
-    //      products are contiguous in sOrd (ascending tile, then k); their
-    //      indices are read 32 at a time, one per lane, and broadcast, so a
-    //      product costs no dependent shared-memory lookups; kPushDepth B
-    //      tiles in flight ----
+    //      products are contiguous in sOrd (ascending tile, then k) ----
+    const int t0 = (nt * warp) / WARPS, t1 = (nt * (warp + 1)) / WARPS;
+    const int q0 = t0 ? sCnt[t0 - 1] : 0, q1 = t1 ? sCnt[t1 - 1] : 0;
     const int gq = lane >> 2, tq = lane & 3;
-    const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA);
-    const uint32_t slots = (uint32_t)__cvta_generic_to_shared(sB + warp * kPushDepth * 512);
-    const int swz = tile_swz(lane >> 1, lane & 1);
-    const int t0 = (nt * warp) / kRowWarps, t1 = (nt * (warp + 1)) / kRowWarps;
-    if (t0 < t1)
+    const bool f32 = p.out_type == KAMI_F32, bf = p.out_type == KAMI_BF16;
+    const bool plain = p.alpha == 1.f && p.beta == 0.f && !(reinterpret_cast<uintptr_t>(p.vc) & (f32 ? 15 : 7));
+    uint8_t *const out = reinterpret_cast<uint8_t *>(p.vc) + ((int64_t)c0 * 256 + gq * 16 + 4 * tq) * (f32 ? 4 : 2);
+    // tiles without products hold zeros
+    for (int base = t0; base < t1; base += 32)
     {
-        const int q0 = t0 ? sCnt[t0 - 1] : 0, q1 = sCnt[t1 - 1]; // this warp's products
-        // product q's (A entry << 16 | tile) and B entry, for q = base + lane
-        auto load_info = [&](int base, int &pep, int &pb) {
-            const int q = base + lane;
-            pep = 0;
-            pb = 0;
-            if (q < q1)
-            {
-                const int f = sOrd[q];
-                pep = sPep[f];
-                pb = sPb[f];
-            }
-        };
-        int ib = q0, i_pep, i_pb; // issue side: info chunk at ib
-        load_info(ib, i_pep, i_pb);
-        int qi = q0, issued = 0;
-        auto issue = [&]() {
-            if (qi < q1)
-            {
-                if (qi - ib >= 32)
-                {
-                    ib += 32;
-                    load_info(ib, i_pep, i_pb);
-                }
-                const int eb = __shfl_sync(0xffffffffu, i_pb, qi - ib);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slots + (issued % kPushDepth) * 512 +
-                                                                                swz),
-                             "l"(p.vb + (int64_t)eb * 256 + lane * 8)
-                             : "memory");
-                ++qi;
-                ++issued;
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-#pragma unroll
-        for (int d = 0; d < kPushDepth - 1; ++d)
-            issue();
-        int cb = q0, c_pep, c_pb; // consumer side: info chunk at cb
-        load_info(cb, c_pep, c_pb);
-        float acc0[4] = {0.f, 0.f, 0.f, 0.f};
-        float acc1[4] = {0.f, 0.f, 0.f, 0.f};
-        int tile = t0;
-        for (int qc = q0; qc < q1; ++qc)
+        const int t = base + lane;
+        unsigned none = __ballot_sync(0xffffffffu, t < t1 && sCnt[t] == (t ? sCnt[t - 1] : 0));
+        for (; none; none &= none - 1)
+            push_store(p, c0 + base + __ffs(none) - 1, gq, tq, make_float4(0.f, 0.f, 0.f, 0.f),
+                       make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    const uint32_t a_lane = tile_ldsm_addr((uint32_t)__cvta_generic_to_shared(sA), lane);
+    const uint8_t *const b_lane = reinterpret_cast<const uint8_t *>(p.vb) + tq * 64 + gq * 4;
+    float acc0[4] = {0.f, 0.f, 0.f, 0.f}; // columns 4 tq, 4 tq + 2
+    float acc1[4] = {0.f, 0.f, 0.f, 0.f}; // columns 4 tq + 1, 4 tq + 3
+    uint32_t nx[kPushDepth][4];           // rows 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9 of the next products' B tiles
+    for (int base = q0; base < q1; base += 32)
+    {
+        // lane l: product base + l, as its A tile's place, its C tile (bit 31:
+        // the last product of that tile) and its B entry
+        const int n = min(32, q1 - base);
+        int place = 0, tile = 0, eb = 0;
+        if (lane < n)
         {
-            issue(); // kPushDepth - 1 products ahead, into the slot read last
-            if (qc - cb >= 32)
-            {
-                cb += 32;
-                load_info(cb, c_pep, c_pb);
-            }
-            const int pep = __shfl_sync(0xffffffffu, c_pep, qc - cb);
-            const int pt = pep & 0xffff, e = pep >> 16;
-            while (tile < pt) // the previous tile is complete (tiles without products store zeros)
-            {
-                store_c_tile(p, (int64_t)c0 + tile, gq, tq, acc0, acc1);
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    acc0[x] = acc1[x] = 0.f;
-                ++tile;
-            }
-            asm volatile("cp.async.wait_group %0;" ::"n"(kPushDepth - 1) : "memory");
-            __syncwarp();
-            uint32_t a[4], b[4];
-            ldsm4(tile_ldsm_addr(sA_u + e * 512, lane), a);
-            ldsm4_t(tile_ldsm_addr(slots + ((qc - q0) % kPushDepth) * 512, lane), b);
-            for (int r = 0; r < p.num_iter; ++r)
-            {
-                mma16816<BF16>(acc0, a[0], a[1], a[2], a[3], b[0], b[1]);
-                mma16816<BF16>(acc1, a[0], a[1], a[2], a[3], b[2], b[3]);
-            }
-            __syncwarp(); // every lane's fragments are read before the slot is refilled
+            const int f = sOrd[base + lane], pep = sPep[f];
+            place = (pep >> 16) * 512;
+            tile = pep & 0xffff;
+            if (base + lane + 1 == sCnt[tile])
+                tile |= (int)0x80000000;
+            eb = sPb[f];
         }
-        for (; tile < t1; ++tile)
-        {
-            store_c_tile(p, (int64_t)c0 + tile, gq, tq, acc0, acc1);
+        auto fetch = [&](int x, uint32_t(&v)[4]) {
+            const uint8_t *const b = b_lane + (int64_t)__shfl_sync(0xffffffffu, eb, x) * 512;
+            v[0] = __ldg(reinterpret_cast<const uint32_t *>(b));
+            v[1] = __ldg(reinterpret_cast<const uint32_t *>(b + 32));
+            v[2] = __ldg(reinterpret_cast<const uint32_t *>(b + 256));
+            v[3] = __ldg(reinterpret_cast<const uint32_t *>(b + 288));
+        };
 #pragma unroll
-            for (int x = 0; x < 4; ++x)
-                acc0[x] = acc1[x] = 0.f;
+        for (int d = 0; d < kPushDepth; ++d)
+            fetch(min(d, n - 1), nx[d]);
+        for (int x = 0; x < n; x += kPushDepth)
+        {
+#pragma unroll
+            for (int d = 0; d < kPushDepth; ++d)
+                if (x + d < n)
+                {
+                    uint32_t a[4];
+                    ldsm4(a_lane + __shfl_sync(0xffffffffu, place, x + d), a);
+                    const int t = __shfl_sync(0xffffffffu, tile, x + d);
+                    // low halves: column 2 gq of two rows; high halves: column 2 gq + 1
+                    const uint32_t e0 = __byte_perm(nx[d][0], nx[d][1], 0x5410), o0 = __byte_perm(nx[d][0], nx[d][1], 0x7632);
+                    const uint32_t e1 = __byte_perm(nx[d][2], nx[d][3], 0x5410), o1 = __byte_perm(nx[d][2], nx[d][3], 0x7632);
+                    fetch(min(x + d + kPushDepth, n - 1), nx[d]);
+                    for (int r = 0; r < p.num_iter; ++r)
+                    {
+                        mma16816<BF16>(acc0, a[0], a[1], a[2], a[3], e0, e1);
+                        mma16816<BF16>(acc1, a[0], a[1], a[2], a[3], o0, o1);
+                    }
+                    if (t < 0)
+                    {
+                        const float4 lo = make_float4(acc0[0], acc1[0], acc0[1], acc1[1]);
+                        const float4 hi = make_float4(acc0[2], acc1[2], acc0[3], acc1[3]);
+                        if (plain && f32)
+                        {
+                            float4 *const o = reinterpret_cast<float4 *>(out + (int64_t)(t & 0xffff) * 1024);
+                            o[0] = lo;
+                            o[32] = hi;
+                        }
+                        else if (plain)
+                        {
+                            uint2 *const o = reinterpret_cast<uint2 *>(out + (int64_t)(t & 0xffff) * 512);
+                            o[0] = make_uint2(pack16(lo.x, lo.y, bf), pack16(lo.z, lo.w, bf));
+                            o[32] = make_uint2(pack16(hi.x, hi.y, bf), pack16(hi.z, hi.w, bf));
+                        }
+                        else
+                            push_store(p, c0 + (t & 0xffff), gq, tq, lo, hi);
+#pragma unroll
+                        for (int y = 0; y < 4; ++y)
+                            acc0[y] = acc1[y] = 0.f;
+                    }
+                }
         }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+template <bool BF16, bool FILL> void push_launch(const SpNumArgs &p, bool few, cudaStream_t s)
+{
+    if (few)
+        spgemm_numeric_push_kernel<BF16, FILL, kPushWarpsFew><<<(unsigned)p.mb, kPushWarpsFew * 32, 0, s>>>(p);
+    else
+        spgemm_numeric_push_kernel<BF16, FILL, kPushWarps><<<(unsigned)p.mb, kPushWarps * 32, 0, s>>>(p);
+}
+
+void push_launch(const SpNumArgs &p, bool bf16, bool fill, bool few, cudaStream_t s)
+{
+    if (bf16)
+        fill ? push_launch<true, true>(p, few, s) : push_launch<true, false>(p, few, s);
+    else
+        fill ? push_launch<false, true>(p, few, s) : push_launch<false, false>(p, few, s);
 }
 
 int bitmap_launch(int nb, int *warps_per_cta, size_t *smem)
@@ -1441,11 +1579,12 @@ int kami_spgemm_bsr_numeric(kami_dtype_t in_type, kami_dtype_t out_type, int bsr
                                            val_c, nnz_c, alpha, beta, num_iter, stream);
 }
 
-int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr,
-                                    int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
-                                    const void *val_a, const int *row_ptr_b, const int *col_idx_b, const void *val_b,
-                                    const int *row_ptr_c, const int *col_idx_c, void *val_c, int64_t nnz_c,
-                                    double alpha, double beta, int num_iter, void *stream)
+// The numeric pass; fill: ColIdxC is written too (col_idx_c is then an output).
+static int numeric_pass(bool fill, kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr,
+                        int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
+                        const void *val_a, const int *row_ptr_b, const int *col_idx_b, const void *val_b,
+                        const int *row_ptr_c, int *col_idx_c, void *val_c, int64_t nnz_c,
+                        double alpha, double beta, int num_iter, void *stream)
 {
     if (variant != KAMI_VARIANT_AUTO && variant != KAMI_VARIANT_MMA_SYNC && variant != KAMI_VARIANT_TCGEN05)
         return fail(KAMI_ERR_INVALID_VALUE, "spgemm numeric: variant must be AUTO, MMA_SYNC or TCGEN05");
@@ -1474,7 +1613,7 @@ int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type
     p.rpb = row_ptr_b;
     p.cib = col_idx_b;
     p.rpc = row_ptr_c;
-    p.cic = col_idx_c;
+    p.cic = p.cic_out = col_idx_c;
     p.va = reinterpret_cast<const uint16_t *>(val_a);
     p.vb = reinterpret_cast<const uint16_t *>(val_b);
     p.vc = val_c;
@@ -1491,16 +1630,21 @@ int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type
     const bool tc_ok = aligned16 && !(reinterpret_cast<uintptr_t>(val_c) & 15);
     if (variant == KAMI_VARIANT_TCGEN05 && !tc_ok)
         return fail(KAMI_ERR_MISALIGNED, "spgemm numeric (tcgen05): tile arrays must be 16-byte aligned");
-    if (variant == KAMI_VARIANT_TCGEN05 || (variant == KAMI_VARIANT_AUTO && tc_ok && spgemm_auto_tc05()))
+    const bool tc = variant == KAMI_VARIANT_TCGEN05 || (variant == KAMI_VARIANT_AUTO && tc_ok && spgemm_auto_tc05());
+    // the push kernel fills ColIdxC itself, up to 16384 block columns
+    const bool with = fill && !tc && aligned16 && nb <= kFillWords * 32;
+    if (fill && !with && (st = kami_spgemm_bsr_fill_colidx(bsr, mb, kb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b,
+                                                           row_ptr_c, col_idx_c, stream)))
+        return st;
+    if (tc)
         return spgemm_tc05_launch(in_type == KAMI_BF16, mb, nnz_c, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b, row_ptr_c,
                                   col_idx_c, val_a, val_b, val_c, out_type, alpha, beta, num_iter, s);
-    const bool rowwise = aligned16;
-    if (rowwise) // one CTA per block-row, staged operands, products pushed to their tiles
+    if (aligned16) // one CTA per block-row, products pushed to their tiles
     {
-        if (in_type == KAMI_BF16)
-            spgemm_numeric_push_kernel<true><<<(unsigned)mb, kPushWarps * 32, 0, s>>>(p);
-        else
-            spgemm_numeric_push_kernel<false><<<(unsigned)mb, kPushWarps * 32, 0, s>>>(p);
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        push_launch(p, in_type == KAMI_BF16, with, mb <= kPushFewPerSm * sms, s);
     }
     else if (in_type == KAMI_BF16)
         spgemm_numeric_kernel<true><<<(unsigned)grid, 256, 0, s>>>(p);
@@ -1510,6 +1654,27 @@ int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type
     if (e != cudaSuccess)
         return cuda_fail(e, "spgemm_numeric_kernel");
     return KAMI_OK;
+}
+
+int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr,
+                                    int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
+                                    const void *val_a, const int *row_ptr_b, const int *col_idx_b, const void *val_b,
+                                    const int *row_ptr_c, const int *col_idx_c, void *val_c, int64_t nnz_c,
+                                    double alpha, double beta, int num_iter, void *stream)
+{
+    return numeric_pass(false, variant, in_type, out_type, bsr, mb, kb, nb, row_ptr_a, col_idx_a, val_a, row_ptr_b,
+                        col_idx_b, val_b, row_ptr_c, const_cast<int *>(col_idx_c), val_c, nnz_c, alpha, beta, num_iter,
+                        stream);
+}
+
+int kami_spgemm_bsr_fill_numeric(kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr, int mb,
+                                 int kb, int nb, const int *row_ptr_a, const int *col_idx_a, const void *val_a,
+                                 const int *row_ptr_b, const int *col_idx_b, const void *val_b, const int *row_ptr_c,
+                                 int *col_idx_c, void *val_c, int64_t nnz_c, double alpha, double beta, int num_iter,
+                                 void *stream)
+{
+    return numeric_pass(true, variant, in_type, out_type, bsr, mb, kb, nb, row_ptr_a, col_idx_a, val_a, row_ptr_b,
+                        col_idx_b, val_b, row_ptr_c, col_idx_c, val_c, nnz_c, alpha, beta, num_iter, stream);
 }
 
 } // extern "C"

@@ -37,8 +37,7 @@ using at::Tensor;
 decltype(&kami_gemm_batched) g_gemm = nullptr;
 decltype(&kami_spmm_bsr) g_spmm = nullptr;
 decltype(&kami_spgemm_bsr_symbolic) g_symbolic = nullptr;
-decltype(&kami_spgemm_bsr_fill_colidx) g_fill = nullptr;
-decltype(&kami_spgemm_bsr_numeric_variant) g_numeric = nullptr;
+decltype(&kami_spgemm_bsr_fill_numeric) g_fill_numeric = nullptr;
 
 // What Python has to look at itself.
 struct Decline
@@ -268,23 +267,23 @@ PyObject *spgemm(PyObject *, PyObject *const *a, Py_ssize_t n)
         const void *pva = entries(va), *pvb = entries(vb);
         int *prc = static_cast<int *>(rc.data_ptr());
         void *stream = c10::cuda::getCurrentCUDAStream(ra.device().index()).stream();
-        int nnz = 0;
-        int st = unlocked([&] { return g_symbolic(16, mb, kb, nb, pra, pca, prb, pcb, prc, &nnz, stream); });
+        // page-locked, so that its copy is one transfer (torch keeps and reuses the block)
+        const Tensor count = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+        int *pn = static_cast<int *>(count.data_ptr());
+        int st = unlocked([&] { return g_symbolic(16, mb, kb, nb, pra, pca, prb, pcb, prc, pn, stream); });
         if (st != KAMI_OK)
             return PyLong_FromLong(st);
+        const int nnz = *pn;
         const int64_t room = nnz > 0 ? nnz : 1;
         const Tensor cc = at::empty({room}, ints);
         int *pcc = static_cast<int *>(cc.data_ptr());
-        st = unlocked([&] { return g_fill(16, mb, kb, nb, pra, pca, prb, pcb, prc, pcc, stream); });
-        if (st != KAMI_OK)
-            return PyLong_FromLong(st);
         const Tensor vc = at::empty({room, 16, 16}, ints.dtype(o));
         void *pvc = vc.data_ptr();
         int *pcn = nnz > 0 ? pcc : nullptr;
         if (nnz <= 0)
             pvc = nullptr;
         st = unlocked([&] {
-            return g_numeric((kami_variant_t)variant, (kami_dtype_t)in, (kami_dtype_t)out, 16, mb, kb, nb, pra, pca, pva,
+            return g_fill_numeric((kami_variant_t)variant, (kami_dtype_t)in, (kami_dtype_t)out, 16, mb, kb, nb, pra, pca, pva,
                              prb, pcb, pvb, prc, pcn, pvc, nnz, 1.0, 0.0, iters, stream);
         });
         if (st != KAMI_OK)
@@ -299,18 +298,17 @@ PyObject *spgemm(PyObject *, PyObject *const *a, Py_ssize_t n)
     });
 }
 
-// bind(kami_gemm_batched, kami_spmm_bsr, kami_spgemm_bsr_symbolic, kami_spgemm_bsr_fill_colidx,
-//      kami_spgemm_bsr_numeric_variant): their addresses in the loaded library
+// bind(kami_gemm_batched, kami_spmm_bsr, kami_spgemm_bsr_symbolic, kami_spgemm_bsr_fill_numeric): their addresses
+// in the loaded library
 PyObject *bind(PyObject *, PyObject *args)
 {
-    unsigned long long p[5];
-    if (!PyArg_ParseTuple(args, "KKKKK", &p[0], &p[1], &p[2], &p[3], &p[4]))
+    unsigned long long p[4];
+    if (!PyArg_ParseTuple(args, "KKKK", &p[0], &p[1], &p[2], &p[3]))
         return nullptr;
     g_gemm = reinterpret_cast<decltype(g_gemm)>(p[0]);
     g_spmm = reinterpret_cast<decltype(g_spmm)>(p[1]);
     g_symbolic = reinterpret_cast<decltype(g_symbolic)>(p[2]);
-    g_fill = reinterpret_cast<decltype(g_fill)>(p[3]);
-    g_numeric = reinterpret_cast<decltype(g_numeric)>(p[4]);
+    g_fill_numeric = reinterpret_cast<decltype(g_fill_numeric)>(p[3]);
     Py_RETURN_NONE;
 }
 
