@@ -57,6 +57,7 @@
 
 #include "grouped.cuh"
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "ring.cuh"
 #include "tc05_ptx.cuh"
 
@@ -386,6 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_ring_kernel(const __grid_cons
         tc::mbar_init(&empty[lane], kWarps);
         tc::fence_mbar_init();
     }
+    wait_for_previous();
     // this CTA's chunks: a plan's list, or a share of the batch's parts
     int64_t first;
     int n, stride = 1;
@@ -499,7 +501,7 @@ int launch_ring(const RingParams &rp, int ctas, cudaStream_t s)
     if (attr[dev] != cudaSuccess)
         return cuda_fail(attr[dev], "cudaFuncSetAttribute(f64_ring_kernel)");
     void *args[] = {const_cast<RingParams *>(&rp)};
-    e = cudaLaunchKernel((const void *)&f64_ring_kernel, dim3(ctas), dim3(kThreads), args, kSmem, s);
+    e = launch_overlapped((const void *)&f64_ring_kernel, dim3(ctas), dim3(kThreads), args, kSmem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(f64_ring_kernel)");
     return KAMI_OK;

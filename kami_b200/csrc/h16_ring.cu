@@ -38,6 +38,7 @@
 
 #include "grouped.cuh"
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "ring.cuh"
 #include "tc05_epi.cuh"
 #include "tc05_ptx.cuh"
@@ -378,6 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
         tc::tmem_alloc(tmem_slot, 128 * kGroups);
         tc::tmem_relinquish();
     }
+    wait_for_previous();
     // the group's chunks: a plan's list, or every so many-th problem of the batch
     const int worker = g * gridDim.x + blockIdx.x, workers = gridDim.x * kGroups;
     int64_t first;
@@ -543,7 +545,7 @@ int launch_ring(const RingParams &rp, bool bf16, int ctas, cudaStream_t s)
     if (attr[dev][bf16] != cudaSuccess)
         return cuda_fail(attr[dev][bf16], "cudaFuncSetAttribute(h16_ring_kernel)");
     void *args[] = {const_cast<RingParams *>(&rp)};
-    e = cudaLaunchKernel(ring_fn(bf16), dim3(ctas), dim3(kThreads), args, kSmem, s);
+    e = launch_overlapped(ring_fn(bf16), dim3(ctas), dim3(kThreads), args, kSmem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(h16_ring_kernel)");
     return KAMI_OK;

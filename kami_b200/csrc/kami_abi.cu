@@ -520,8 +520,8 @@ int gemm_batched_hinted(kami_dtype_t in_type, kami_dtype_t out_type, kami_partit
         gc.C = reinterpret_cast<char *>(g.C) + first * g.sC * osz;
         gc.batch = g.batch - first;
         params[0] = &gc;
-        cudaError_t e = cudaLaunchKernel(inst->fn, dim3((unsigned)chunk), dim3(info.threads), params,
-                                         (size_t)info.smem, s);
+        cudaError_t e = launch_overlapped(inst->fn, dim3((unsigned)chunk), dim3(info.threads), params,
+                                          (size_t)info.smem, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaLaunchKernel(block_mma_kernel)");
         done += chunk;

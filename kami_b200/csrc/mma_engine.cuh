@@ -53,6 +53,7 @@
 #pragma once
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 
 namespace kami {
 
@@ -263,6 +264,7 @@ __global__ void block_mma_kernel(const GemmArgs g)
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
 
+    wait_for_previous();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int group = warp / G::NW;

@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "spgemm_tiles.cuh"
 
 namespace kami {
@@ -89,6 +90,7 @@ __global__ void spgemm_count_kernel(int mb, int nb, const int *__restrict__ rpa,
                                     const int *__restrict__ rpb, const int *__restrict__ cib, int *__restrict__ rpc)
 {
     extern __shared__ uint32_t bm_all[];
+    wait_for_previous();
     const int words = (nb + 31) >> 5;
     const int wpc = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(1024) spgemm_scan_kernel(int n, int *__restric
     __shared__ int warp_sums[32];
     __shared__ int carry_s;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    wait_for_previous();
     if (t == 0)
         carry_s = 0;
     __syncthreads();
@@ -984,6 +987,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     __shared__ int sOff[kPushMaxA + 1];
     __shared__ int sK[kPushMaxA];
     __shared__ int sRb[kPushMaxA];
+    wait_for_previous();
     const int i = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int kT = WARPS * 32;
@@ -1248,20 +1252,19 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     }
 }
 
-template <bool BF16, bool FILL> void push_launch(const SpNumArgs &p, bool few, cudaStream_t s)
+template <bool BF16, bool FILL> cudaError_t push_launch(const SpNumArgs &p, bool few, cudaStream_t s)
 {
-    if (few)
-        spgemm_numeric_push_kernel<BF16, FILL, kPushWarpsFew><<<(unsigned)p.mb, kPushWarpsFew * 32, 0, s>>>(p);
-    else
-        spgemm_numeric_push_kernel<BF16, FILL, kPushWarps><<<(unsigned)p.mb, kPushWarps * 32, 0, s>>>(p);
+    const void *fn = few ? (const void *)spgemm_numeric_push_kernel<BF16, FILL, kPushWarpsFew>
+                         : (const void *)spgemm_numeric_push_kernel<BF16, FILL, kPushWarps>;
+    void *args[] = {const_cast<SpNumArgs *>(&p)};
+    return launch_overlapped(fn, dim3((unsigned)p.mb), dim3(32 * (few ? kPushWarpsFew : kPushWarps)), args, 0, s);
 }
 
-void push_launch(const SpNumArgs &p, bool bf16, bool fill, bool few, cudaStream_t s)
+cudaError_t push_launch(const SpNumArgs &p, bool bf16, bool fill, bool few, cudaStream_t s)
 {
     if (bf16)
-        fill ? push_launch<true, true>(p, few, s) : push_launch<true, false>(p, few, s);
-    else
-        fill ? push_launch<false, true>(p, few, s) : push_launch<false, false>(p, few, s);
+        return fill ? push_launch<true, true>(p, few, s) : push_launch<true, false>(p, few, s);
+    return fill ? push_launch<false, true>(p, few, s) : push_launch<false, false>(p, few, s);
 }
 
 int bitmap_launch(int nb, int *warps_per_cta, size_t *smem)
@@ -1476,12 +1479,12 @@ int kami_spgemm_bsr_symbolic(int bsr, int mb, int kb, int nb, const int *row_ptr
         if ((st = prep_bitmap_fn((const void *)spgemm_count_kernel, smem)))
             return st;
         const int grid = (mb + wpc - 1) / wpc;
-        spgemm_count_kernel<<<grid, wpc * 32, smem, s>>>(mb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b,
-                                                        row_ptr_c);
-        if ((e = cudaGetLastError()) != cudaSuccess)
+        void *count_args[] = {&mb, &nb, &row_ptr_a, &col_idx_a, &row_ptr_b, &col_idx_b, &row_ptr_c};
+        if ((e = launch_overlapped((const void *)spgemm_count_kernel, dim3(grid), dim3(wpc * 32), count_args, smem, s)) !=
+            cudaSuccess)
             return cuda_fail(e, "spgemm_count_kernel");
-        spgemm_scan_kernel<<<1, 1024, 0, s>>>(mb, row_ptr_c);
-        if ((e = cudaGetLastError()) != cudaSuccess)
+        void *scan_args[] = {&mb, &row_ptr_c};
+        if ((e = launch_overlapped((const void *)spgemm_scan_kernel, dim3(1), dim3(1024), scan_args, 0, s)) != cudaSuccess)
             return cuda_fail(e, "spgemm_scan_kernel");
     }
     else
@@ -1644,9 +1647,10 @@ static int numeric_pass(bool fill, kami_variant_t variant, kami_dtype_t in_type,
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        push_launch(p, in_type == KAMI_BF16, with, mb <= kPushFewPerSm * sms, s);
+        const cudaError_t el = push_launch(p, in_type == KAMI_BF16, with, mb <= kPushFewPerSm * sms, s);
+        return el == cudaSuccess ? KAMI_OK : cuda_fail(el, "spgemm_numeric_push_kernel");
     }
-    else if (in_type == KAMI_BF16)
+    if (in_type == KAMI_BF16)
         spgemm_numeric_kernel<true><<<(unsigned)grid, 256, 0, s>>>(p);
     else
         spgemm_numeric_kernel<false><<<(unsigned)grid, 256, 0, s>>>(p);

@@ -38,6 +38,7 @@
 #include <mutex>
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "tc05_ptx.cuh"
 
 namespace kami {
@@ -934,6 +935,7 @@ __global__ void __launch_bounds__(persistent_threads<SK, S>(), 1) split_f64_pers
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    wait_for_previous();
 
     if (warp < kSplitWarps)
     {
@@ -1301,7 +1303,7 @@ extern "C" int kami_split_f64_gemm_batched(int nslices, kami_dtype_t slice_type,
             return cuda_fail(e2, "cudaFuncSetAttribute(split_f64_persistent)");
         const int64_t grid = batch < sms ? batch : sms;
         void *args2[] = {&sp, &mapA, &mapB};
-        e2 = cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)fns.persistent_threads), args2, smem, st);
+        e2 = launch_overlapped(fn, dim3((unsigned)grid), dim3((unsigned)fns.persistent_threads), args2, smem, st);
         if (e2 != cudaSuccess)
             return cuda_fail(e2, "cudaLaunchKernel(split_f64_persistent)");
         return KAMI_OK;

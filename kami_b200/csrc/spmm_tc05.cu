@@ -45,6 +45,7 @@
 #include <mutex>
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "tc05_ptx.cuh"
 
 namespace kami {
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) spmm_tc05_kernel(const _
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    wait_for_previous();
 
     if (warp == 0 || warp == kLoadWarp2)
     {
@@ -455,7 +457,7 @@ int spmm_tc05_launch(bool bf16, int out_type, int mb, int kb, int N, const int *
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = mb < sms * kCtasPerSm ? mb : sms * kCtasPerSm;
     void *args[] = {&map, &p};
-    e = cudaLaunchKernel(kfn, dim3(grid), dim3(kThreads), args, smem, s);
+    e = launch_overlapped(kfn, dim3(grid), dim3(kThreads), args, smem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(spmm_tc05_kernel)");
     return KAMI_OK;

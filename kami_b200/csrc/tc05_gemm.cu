@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 #include "tc05_epi.cuh"
 #include "tc05_gemm.cuh"
 #include "tc05_ptx.cuh"
@@ -552,6 +553,7 @@ __global__ void __launch_bounds__(96 + 128 * kStreamMaxGroups, 1) tc05_stream_ke
         tc::fence_mbar_init();
         // every slot is free: the first loads start before the TMEM
         // allocation and the block barrier
+        wait_for_previous();
         for (int64_t prob = blockIdx.x; prob < nunit && j0 < S; prob += gridDim.x, ++j0)
             load_slot(j0, prob);
     }
@@ -566,6 +568,7 @@ __global__ void __launch_bounds__(96 + 128 * kStreamMaxGroups, 1) tc05_stream_ke
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint64_t limit = p.timeout_ns;
+    wait_for_previous();
 
     if (warp == 0)
     {
@@ -1136,8 +1139,8 @@ static int stream_launch(CUtensorMap &ma, CUtensorMap &mb, Tc05Params &p, bool b
     if (need_two && sp.issuers != 2)
         return KAMI_ERR_UNSUPPORTED; // nothing launched: the caller runs one CTA per problem
     void *args[] = {&ma, &mb, &mc, &sp};
-    e = cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(64 + 128 * sp.groups + 32 * (sp.issuers - 1)), args, smem,
-                         stream);
+    e = launch_overlapped(fn, dim3((unsigned)grid), dim3(64 + 128 * sp.groups + 32 * (sp.issuers - 1)), args, smem,
+                          stream);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(tc05_stream_kernel)");
     return KAMI_OK;
@@ -1308,6 +1311,7 @@ __global__ void __launch_bounds__(128) tc05_bwd_kernel(const __grid_constant__ C
         tc::prefetch_tmap(&tmA);
         tc::prefetch_tmap(&tmB);
         tc::mbar_expect_tx(&bars[0], (uint32_t)((M * N + M * K + K * N) * 2 * nq));
+        wait_for_previous();
         for (int q = 0; q < nq; ++q)
         {
             const int pr = (p.pair ? 2 * blockIdx.x : blockIdx.x) + q;
@@ -1328,6 +1332,7 @@ __global__ void __launch_bounds__(128) tc05_bwd_kernel(const __grid_constant__ C
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
+    wait_for_previous();
     const uint32_t tmem = *tmem_slot;
 
     if (threadIdx.x == 0)
@@ -1502,7 +1507,7 @@ int tc05_backward_launch(int in_type, int out_type, int M, int N, int K, int64_t
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaFuncSetAttribute(tc05_bwd_kernel)");
     void *args[] = {&mg, &ma, &mb, &mda, &mdb, &p};
-    e = cudaLaunchKernel(fn, dim3((unsigned)(p.pair ? (batch + 1) / 2 : batch)), dim3(128), args, smem, stream);
+    e = launch_overlapped(fn, dim3((unsigned)(p.pair ? (batch + 1) / 2 : batch)), dim3(128), args, smem, stream);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(tc05_bwd_kernel)");
     return KAMI_OK;
