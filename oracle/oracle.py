@@ -45,7 +45,7 @@ def build_reference(ref_root: str | None = None) -> bool:
     sources are present (``ref_root``, default :func:`reference_root`).
     Returns True when the libraries exist afterwards."""
     ref_root = ref_root or reference_root()
-    if os.path.isdir(ref_root):
+    if os.path.isdir(os.path.join(ref_root, "src")):
         subprocess.run(["make", "-s", "-C", HERE, "-f", "Makefile.ref", "-j8", f"REF={ref_root}"],
                        check=True)
     return os.path.exists(os.path.join(REF_DIR, "libref_spgemm2d_host.so"))
