@@ -5,9 +5,9 @@
 // checks of each tensor, torch.empty, the ctypes conversion of 27 arguments),
 // 3 us of them the launch: more than the kernel of a small batch takes.  Here
 // the same checks and the same call take 3.5 us (1024 x 32^3 FP64, back to
-// back: 11.7 us a call before, 8.2 now).  api.spgemm, whose host waits for the
-// number of C tiles, saves the same on each of its three calls (n = 16384 at
-// 1 %: 83 us before, 71 now).
+// back: 11.7 us a call before, 8.2 after).  api.spgemm, whose host waits for the
+// number of C tiles, saves the same on each of its calls (n = 16384 at 1 %: 83 us
+// before, 71 after).
 //
 // Each function takes the calls it can make as they are and returns what the
 // Python function returns; a failed call returns its status, for the caller to
