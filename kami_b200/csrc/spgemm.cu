@@ -875,12 +875,14 @@ __device__ __forceinline__ void numeric_row_pull(const SpNumArgs &p, const int i
 // ---------------------------------------------------------------------------
 // Warps of a CTA: eight while every block-row has a place at once (four CTAs of
 // eight warps per SM), so that a row takes less time (numeric pass of 300 rows
-// of 9 entries 13.9 us against 17.1, 128 rows 13.0 against 17.1); four past that
-// (4096 rows of 6 48 us against 63, 1024 rows of 10 34.4 against 35.1).
-constexpr int kPushWarps = 4, kPushWarpsFew = 8, kPushFewPerSm = 4;
-constexpr int kPushMaxC = 512;    // C tiles of a row
-constexpr int kPushMaxProd = 512; // products of a row
-constexpr int kPushMaxA = 24;     // A tiles of a row staged (12 KB)
+// of 9 entries 13.9 us against 17.1, 128 rows 13.0 against 17.1), and where rows have
+// 96 C tiles or more on average (1024 rows of 12 entries, 134 tiles: 39 us against 45; of
+// 20, 330 tiles: 196 against 425, as more of them fit the wider staging); four
+// otherwise (4096 rows of 8, 64 tiles: 72 us against 81).
+constexpr int kPushWarps = 4, kPushWarpsMany = 8, kPushFewPerSm = 4, kPushManyTiles = 96;
+// What a CTA of so many warps stages of a row: A tiles (a lane each), C tiles, products
+template <int WARPS> constexpr int kPushMaxA = WARPS == kPushWarpsMany ? 32 : 24;
+template <int WARPS> constexpr int kPushMaxC = WARPS == kPushWarpsMany ? 896 : 512;
 constexpr int kPushDepth = 4;     // B tiles on their way per warp, in registers
 constexpr int kFillWords = 512;   // FILL: words of 32 block columns
 
@@ -972,7 +974,8 @@ __device__ __forceinline__ void row_columns(const uint32_t *bm, int words, int *
 template <bool BF16, bool FILL, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const __grid_constant__ SpNumArgs p)
 {
-    __shared__ __align__(16) uint8_t sA[kPushMaxA * 512];
+    constexpr int MAXA = kPushMaxA<WARPS>, MAXC = kPushMaxC<WARPS>; // products: up to MAXC too
+    __shared__ __align__(16) uint8_t sA[MAXA * 512];
     __shared__ __align__(16) uint8_t sB[WARPS * 512]; // of the per-tile fallback
     __shared__ uint32_t sBits[FILL ? kFillWords : 1];      // the row's columns
     __shared__ int sPre[FILL ? kFillWords : 1];
@@ -980,13 +983,13 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     // entries as its list buffer): the row's ColIdxC, then per tile the
     // product count / range end; per product (A entry << 16) | C position
     // (-1 when absent), its B entry, and the products grouped by C tile
-    __shared__ int sPool[5 * kPushMaxC];
-    static_assert(5 * kPushMaxC >= kMaxBList && kPushMaxProd == kPushMaxC, "fallback list buffer");
-    int *sCol = sPool, *sCnt = sPool + kPushMaxC, *sPep = sPool + 2 * kPushMaxC, *sPb = sPool + 3 * kPushMaxC,
-        *sOrd = sPool + 4 * kPushMaxC;
-    __shared__ int sOff[kPushMaxA + 1];
-    __shared__ int sK[kPushMaxA];
-    __shared__ int sRb[kPushMaxA];
+    __shared__ int sPool[5 * MAXC];
+    static_assert(5 * MAXC >= kMaxBList && MAXA <= 32, "fallback list buffer, a lane per A tile");
+    int *sCol = sPool, *sCnt = sPool + MAXC, *sPep = sPool + 2 * MAXC, *sPb = sPool + 3 * MAXC,
+        *sOrd = sPool + 4 * MAXC;
+    __shared__ int sOff[MAXA + 1];
+    __shared__ int sK[MAXA];
+    __shared__ int sRb[MAXA];
     wait_for_previous();
     const int i = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1001,7 +1004,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     if constexpr (FILL)
         for (int w = tid; w < words; w += kT)
             sBits[w] = 0u;
-    bool pull = nt > kPushMaxC || na > kPushMaxA;
+    bool pull = nt > MAXC || na > MAXA;
     int np = 0;
     if (!pull)
     {
@@ -1040,7 +1043,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
             stage_tile(sA + e * 512, p.va + (int64_t)(a0 + e) * 256, lane);
         __syncthreads();
         np = sOff[na];
-        pull = np > kPushMaxProd;
+        pull = np > MAXC;
     }
     if (pull)
     {
@@ -1057,7 +1060,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
             row_columns(sBits, words, sPre, p.cic_out + c0);
             __syncthreads();
         }
-        numeric_row_pull<BF16, WARPS, kPushMaxA>(p, i, sA, sB, sPool, sOff, sK);
+        numeric_row_pull<BF16, WARPS, MAXA>(p, i, sA, sB, sPool, sOff, sK);
         return;
     }
     // ---- enumerate the products and count them per C tile ----
@@ -1252,19 +1255,19 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     }
 }
 
-template <bool BF16, bool FILL> cudaError_t push_launch(const SpNumArgs &p, bool few, cudaStream_t s)
+template <bool BF16, bool FILL> cudaError_t push_launch(const SpNumArgs &p, bool many, cudaStream_t s)
 {
-    const void *fn = few ? (const void *)spgemm_numeric_push_kernel<BF16, FILL, kPushWarpsFew>
+    const void *fn = many ? (const void *)spgemm_numeric_push_kernel<BF16, FILL, kPushWarpsMany>
                          : (const void *)spgemm_numeric_push_kernel<BF16, FILL, kPushWarps>;
     void *args[] = {const_cast<SpNumArgs *>(&p)};
-    return launch_overlapped(fn, dim3((unsigned)p.mb), dim3(32 * (few ? kPushWarpsFew : kPushWarps)), args, 0, s);
+    return launch_overlapped(fn, dim3((unsigned)p.mb), dim3(32 * (many ? kPushWarpsMany : kPushWarps)), args, 0, s);
 }
 
-cudaError_t push_launch(const SpNumArgs &p, bool bf16, bool fill, bool few, cudaStream_t s)
+cudaError_t push_launch(const SpNumArgs &p, bool bf16, bool fill, bool many, cudaStream_t s)
 {
     if (bf16)
-        return fill ? push_launch<true, true>(p, few, s) : push_launch<true, false>(p, few, s);
-    return fill ? push_launch<false, true>(p, few, s) : push_launch<false, false>(p, few, s);
+        return fill ? push_launch<true, true>(p, many, s) : push_launch<true, false>(p, many, s);
+    return fill ? push_launch<false, true>(p, many, s) : push_launch<false, false>(p, many, s);
 }
 
 int bitmap_launch(int nb, int *warps_per_cta, size_t *smem)
@@ -1647,7 +1650,8 @@ static int numeric_pass(bool fill, kami_variant_t variant, kami_dtype_t in_type,
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const cudaError_t el = push_launch(p, in_type == KAMI_BF16, with, mb <= kPushFewPerSm * sms, s);
+        const cudaError_t el = push_launch(p, in_type == KAMI_BF16, with,
+                                           mb <= kPushFewPerSm * sms || nnz_c >= (int64_t)kPushManyTiles * mb, s);
         return el == cudaSuccess ? KAMI_OK : cuda_fail(el, "spgemm_numeric_push_kernel");
     }
     if (in_type == KAMI_BF16)

@@ -44,6 +44,8 @@ CASES = {  # block-rows, inner, block columns, entries of A's and B's rows
     "few": (40, 30, 70, 4, 5), "many rows": (1200, 20, 33, 2, 3), "one column": (9, 9, 1, 3, 1),
     "A entries": (6, 40, 64, 30, 4), "C tiles": (3, 8, 1100, 6, 200), "products": (5, 24, 100, 20, 60),
     "bitmap full": (12, 10, 16384, 4, 9), "past the bitmap": (12, 10, 16385, 4, 9), "empty rows": (700, 50, 60, 0, 3),
+    "32 A entries": (6, 32, 64, 400, 4), "more A entries": (6, 70, 64, 90, 4), "more C tiles": (3, 8, 2000, 6, 400),
+    "a few long rows": (1200, 90, 60, -1, 4), "long rows": (1200, 40, 200, 9, 30),
 }
 
 
@@ -53,7 +55,7 @@ CASES = {  # block-rows, inner, block columns, entries of A's and B's rows
 def test_fill_and_numeric(cuda, name, dtype, out):
     rows, inner, cols, na, nb = CASES[name]
     rng = np.random.default_rng(len(name))
-    A = _bsr(rng, rows, inner, lambda r: rng.integers(0, inner, (r % 4 == 0) * 3 if na == 0 else na), dtype)
+    A = _bsr(rng, rows, inner, lambda r: rng.integers(0, inner, na if na > 0 else (r % 4 == 0) * 3 if na == 0 else 1 + (r % 50 == 0) * 60), dtype)
     ends = [0, 31, 32, 63, cols - 1]
     B = _bsr(rng, inner, cols, lambda r: [c for c in ends[:1 + r % 5] if c < cols] + list(rng.integers(0, cols, nb)), dtype)
     rp, ci, tiles = _product(rows, A, B)
