@@ -451,7 +451,8 @@ int kami_spgemm_bsr_numeric_variant(kami_variant_t variant, kami_dtype_t in_type
 
 /* kami_spgemm_bsr_fill_colidx and kami_spgemm_bsr_numeric_variant in one call:
  * col_idx_c is written as well (row_ptr_c from kami_spgemm_bsr_symbolic, nnz_c
- * its last entry).  One launch where the block-row kernel runs and nb <= 16384. */
+ * its last entry, or a smaller bound: columns and tiles at or past it are not
+ * written).  One launch where the block-row kernel runs and nb <= 16384. */
 int kami_spgemm_bsr_fill_numeric(kami_variant_t variant, kami_dtype_t in_type, kami_dtype_t out_type, int bsr,
                                  int mb, int kb, int nb,
                                  const int *row_ptr_a, const int *col_idx_a, const void *val_a,

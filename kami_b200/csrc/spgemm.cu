@@ -939,8 +939,8 @@ __device__ __forceinline__ uint32_t pack16(float x, float y, bool bf)
 }
 
 // The row's columns from its bitmap: pre[w] = columns before word w, and
-// ColIdxC's entries.  By the whole CTA.
-__device__ __forceinline__ void row_columns(const uint32_t *bm, int words, int *pre, int *cic)
+// ColIdxC's entries, the first `room` of them.  By the whole CTA.
+__device__ __forceinline__ void row_columns(const uint32_t *bm, int words, int *pre, int *cic, int room)
 {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32)
@@ -966,7 +966,7 @@ __device__ __forceinline__ void row_columns(const uint32_t *bm, int words, int *
     for (int w = threadIdx.x; w < words; w += blockDim.x)
     {
         int at = pre[w];
-        for (uint32_t bits = bm[w]; bits; bits &= bits - 1)
+        for (uint32_t bits = bm[w]; bits && at < room; bits &= bits - 1)
             cic[at++] = w * 32 + __ffs(bits) - 1;
     }
 }
@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
                     atomicOr(&sBits[p.cib[b] >> 5], 1u << (p.cib[b] & 31));
             }
             __syncthreads();
-            row_columns(sBits, words, sPre, p.cic_out + c0);
+            row_columns(sBits, words, sPre, p.cic_out + c0, nt);
             __syncthreads();
         }
         numeric_row_pull<BF16, WARPS, MAXA>(p, i, sA, sB, sPool, sOff, sK);
@@ -1103,10 +1103,15 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
     __syncthreads();
     if constexpr (FILL)
     {
-        row_columns(sBits, words, sPre, p.cic_out + c0);
+        row_columns(sBits, words, sPre, p.cic_out + c0, nt);
         for (int f = tid; f < np; f += kT)
         {
             const int j = sOrd[f], l = sPre[j >> 5] + __popc(sBits[j >> 5] & ((1u << (j & 31)) - 1));
+            if (l >= nt) // a tile past the caller's bound
+            {
+                sPep[f] = -1;
+                continue;
+            }
             sPep[f] |= l;
             atomicAdd(&sCnt[l], 1);
         }
@@ -1505,9 +1510,10 @@ int kami_spgemm_bsr_symbolic(int bsr, int mb, int kb, int nb, const int *row_ptr
     return KAMI_OK;
 }
 
-int kami_spgemm_bsr_fill_colidx(int bsr, int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
-                                const int *row_ptr_b, const int *col_idx_b, const int *row_ptr_c, int *col_idx_c,
-                                void *stream)
+// ColIdxC from RowPtrC, entries at or past `cap` left out.
+static int fill_colidx(int bsr, int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
+                       const int *row_ptr_b, const int *col_idx_b, const int *row_ptr_c, int *col_idx_c, int64_t cap,
+                       void *stream)
 {
     int st = check_bsr_args(bsr, mb, kb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b);
     if (st)
@@ -1524,11 +1530,19 @@ int kami_spgemm_bsr_fill_colidx(int bsr, int mb, int kb, int nb, const int *row_
         return st;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     spgemm_colfill_kernel<<<(mb + wpc - 1) / wpc, wpc * 32, smem, s>>>(mb, nb, row_ptr_a, col_idx_a, row_ptr_b,
-                                                                      col_idx_b, row_ptr_c, col_idx_c, INT64_MAX);
+                                                                      col_idx_b, row_ptr_c, col_idx_c, cap);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_fail(e, "spgemm_colfill_kernel");
     return KAMI_OK;
+}
+
+int kami_spgemm_bsr_fill_colidx(int bsr, int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
+                                const int *row_ptr_b, const int *col_idx_b, const int *row_ptr_c, int *col_idx_c,
+                                void *stream)
+{
+    return fill_colidx(bsr, mb, kb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b, row_ptr_c, col_idx_c, INT64_MAX,
+                       stream);
 }
 
 int kami_spgemm_bsr_symbolic_device(int bsr, int mb, int kb, int nb, const int *row_ptr_a, const int *col_idx_a,
@@ -1639,8 +1653,8 @@ static int numeric_pass(bool fill, kami_variant_t variant, kami_dtype_t in_type,
     const bool tc = variant == KAMI_VARIANT_TCGEN05 || (variant == KAMI_VARIANT_AUTO && tc_ok && spgemm_auto_tc05());
     // the push kernel fills ColIdxC itself, up to 16384 block columns
     const bool with = fill && !tc && aligned16 && nb <= kFillWords * 32;
-    if (fill && !with && (st = kami_spgemm_bsr_fill_colidx(bsr, mb, kb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b,
-                                                           row_ptr_c, col_idx_c, stream)))
+    if (fill && !with && (st = fill_colidx(bsr, mb, kb, nb, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b, row_ptr_c,
+                                           col_idx_c, nnz_c, stream)))
         return st;
     if (tc)
         return spgemm_tc05_launch(in_type == KAMI_BF16, mb, nnz_c, row_ptr_a, col_idx_a, row_ptr_b, col_idx_b, row_ptr_c,
