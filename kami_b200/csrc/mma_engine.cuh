@@ -87,15 +87,15 @@ struct TrH16
     // two units (4 contiguous elements, 8-byte aligned)
     __device__ __forceinline__ static void ld2(const Elem *p, Unit &lo, Unit &hi)
     {
-        uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+        uint2 v = load_operand(reinterpret_cast<const uint2 *>(p));
         lo = v.x;
         hi = v.y;
     }
     // two units gathered from 4 elements at stride s
     __device__ __forceinline__ static void gather2(const Elem *p, int64_t s, Unit &lo, Unit &hi)
     {
-        lo = (uint32_t)__ldg(p) | ((uint32_t)__ldg(p + s) << 16);
-        hi = (uint32_t)__ldg(p + 2 * s) | ((uint32_t)__ldg(p + 3 * s) << 16);
+        lo = (uint32_t)load_operand(p) | ((uint32_t)load_operand(p + s) << 16);
+        hi = (uint32_t)load_operand(p + 2 * s) | ((uint32_t)load_operand(p + 3 * s) << 16);
     }
     __device__ __forceinline__ static void st2(Unit *s, Unit x, Unit y)
     {
@@ -134,14 +134,14 @@ struct TrF64
     }
     __device__ __forceinline__ static void ld2(const Elem *p, Unit &lo, Unit &hi)
     {
-        double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+        double2 v = load_operand(reinterpret_cast<const double2 *>(p));
         lo = v.x;
         hi = v.y;
     }
     __device__ __forceinline__ static void gather2(const Elem *p, int64_t s, Unit &lo, Unit &hi)
     {
-        lo = __ldg(p);
-        hi = __ldg(p + s);
+        lo = load_operand(p);
+        hi = load_operand(p + s);
     }
     __device__ __forceinline__ static void st2(Unit *s, Unit x, Unit y)
     {

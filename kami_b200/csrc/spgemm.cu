@@ -65,9 +65,8 @@ constexpr int kBsr = 16;
 // ---------------------------------------------------------------------------
 // symbolic
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void build_row_bitmap(uint32_t *bm, int words, int row, const int *__restrict__ rpa,
-                                                 const int *__restrict__ cia, const int *__restrict__ rpb,
-                                                 const int *__restrict__ cib, int lane)
+__device__ __forceinline__ void build_row_bitmap(uint32_t *bm, int words, int row, const int *rpa, const int *cia,
+                                                 const int *rpb, const int *cib, int lane)
 {
     for (int w = lane; w < words; w += 32)
         bm[w] = 0u;
@@ -86,8 +85,8 @@ __device__ __forceinline__ void build_row_bitmap(uint32_t *bm, int words, int ro
     __syncwarp();
 }
 
-__global__ void spgemm_count_kernel(int mb, int nb, const int *__restrict__ rpa, const int *__restrict__ cia,
-                                    const int *__restrict__ rpb, const int *__restrict__ cib, int *__restrict__ rpc)
+__global__ void spgemm_count_kernel(int mb, int nb, const int *rpa, const int *cia, const int *rpb, const int *cib,
+                                    int *rpc)
 {
     extern __shared__ uint32_t bm_all[];
     wait_for_previous();
@@ -112,7 +111,7 @@ __global__ void spgemm_count_kernel(int mb, int nb, const int *__restrict__ rpa,
 
 // In-place exclusive scan of rpc[0..n-1] by one CTA of 1024 threads; the
 // total lands in rpc[n].
-__global__ void __launch_bounds__(1024) spgemm_scan_kernel(int n, int *__restrict__ rpc)
+__global__ void __launch_bounds__(1024) spgemm_scan_kernel(int n, int *rpc)
 {
     __shared__ int warp_sums[32];
     __shared__ int carry_s;
@@ -829,10 +828,10 @@ __device__ __forceinline__ void numeric_row_pull(const SpNumArgs &p, const int i
                     else
                     {
                         const uint32_t *ta = reinterpret_cast<const uint32_t *>(p.va + (int64_t)(a0 + ea) * 256);
-                        a[0] = __ldg(ta + (gq * 16 + 2 * tq) / 2);
-                        a[1] = __ldg(ta + ((gq + 8) * 16 + 2 * tq) / 2);
-                        a[2] = __ldg(ta + (gq * 16 + 2 * tq + 8) / 2);
-                        a[3] = __ldg(ta + ((gq + 8) * 16 + 2 * tq + 8) / 2);
+                        a[0] = load_operand(ta + (gq * 16 + 2 * tq) / 2);
+                        a[1] = load_operand(ta + ((gq + 8) * 16 + 2 * tq) / 2);
+                        a[2] = load_operand(ta + (gq * 16 + 2 * tq + 8) / 2);
+                        a[3] = load_operand(ta + ((gq + 8) * 16 + 2 * tq + 8) / 2);
                     }
                     __syncwarp(); // the slot's previous tile has been read
                     stage_tile(slot_p, p.vb + (int64_t)eb * 256, lane);
@@ -1207,10 +1206,10 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
         }
         auto fetch = [&](int x, uint32_t(&v)[4]) {
             const uint8_t *const b = b_lane + (int64_t)__shfl_sync(0xffffffffu, eb, x) * 512;
-            v[0] = __ldg(reinterpret_cast<const uint32_t *>(b));
-            v[1] = __ldg(reinterpret_cast<const uint32_t *>(b + 32));
-            v[2] = __ldg(reinterpret_cast<const uint32_t *>(b + 256));
-            v[3] = __ldg(reinterpret_cast<const uint32_t *>(b + 288));
+            v[0] = load_operand(reinterpret_cast<const uint32_t *>(b));
+            v[1] = load_operand(reinterpret_cast<const uint32_t *>(b + 32));
+            v[2] = load_operand(reinterpret_cast<const uint32_t *>(b + 256));
+            v[3] = load_operand(reinterpret_cast<const uint32_t *>(b + 288));
         };
 #pragma unroll
         for (int d = 0; d < kPushDepth; ++d)

@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include "kami_common.cuh"
+#include "launch.cuh"
 
 namespace kami {
 namespace sptile {
@@ -23,7 +24,7 @@ __device__ __forceinline__ int tile_swz(int r, int c) { return r * 32 + ((c ^ ((
 // Copy one 512-byte tile (16 bytes per lane) into a swizzled shared tile.
 __device__ __forceinline__ void stage_tile(uint8_t *dst, const uint16_t *src, int lane)
 {
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src) + lane);
+    const uint4 v = load_operand(reinterpret_cast<const uint4 *>(src) + lane);
     *reinterpret_cast<uint4 *>(dst + tile_swz(lane >> 1, lane & 1)) = v;
 }
 
