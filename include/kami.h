@@ -226,7 +226,11 @@ int kami_gemm_trace(kami_partition_t partition, int M, int N, int K, int P, int 
  * Describe the kernel kami_gemm_batched would launch (after AUTO resolution):
  * out[0] = variant, out[1] = partition, out[2] = P, out[3] = threads per
  * CTA, out[4] = dynamic shared memory bytes, out[5] = problems per CTA,
- * out[6] = CTAs in the grid.  Host-only; launches nothing.
+ * out[6] = CTAs in the grid, out[7] = 1 for the persistent ring kernels that
+ * AUTO gives small and ragged problems to (then variant is the MMA they issue,
+ * and out[5] the most problems that one CTA walks).  Operands are taken as packed
+ * and aligned, C = A B^T alone (alpha 1, beta 0, one repeat).  Host-only; launches
+ * nothing.
  */
 int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type,
                        kami_partition_t partition, kami_variant_t variant,

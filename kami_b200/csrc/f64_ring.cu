@@ -618,23 +618,9 @@ int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cu
     return launch_ring(rp, ctas, s);
 }
 
-// A uniform batch, A row-major and B N x K, M, N, K <= 128, 16-byte aligned
-// rows and problems (checked by the callers); KAMI_ERR_UNSUPPORTED, nothing
-// launched, where the strides exceed 32 bits.
-int f64_ring_launch(const GemmArgs &g, cudaStream_t s)
+// A uniform batch as the kernel takes it; returns its CTAs.
+static int uniform_params(const GemmArgs &g, Uniform &u)
 {
-    if (g.lda > 0x7fffffff || g.ldb > 0x7fffffff || g.ldc > 0x7fffffff)
-        return fail(KAMI_ERR_UNSUPPORTED, "no kernel for M=%d N=%d K=%d with rows %lld, %lld, %lld apart", g.M, g.N, g.K,
-                    (long long)g.lda, (long long)g.ldb, (long long)g.ldc);
-    RingParams rp{};
-    rp.p.A = g.A;
-    rp.p.B = g.B;
-    rp.p.C = g.C;
-    rp.p.out_type = KAMI_F64;
-    rp.p.alpha = g.alpha;
-    rp.p.beta = g.beta;
-    rp.p.num_iter = g.num_iter;
-    Uniform &u = rp.u;
     u.M = g.M;
     u.N = g.N;
     u.K = g.K;
@@ -664,11 +650,40 @@ int f64_ring_launch(const GemmArgs &g, cudaStream_t s)
     u.ahead0 = std::min(kRecs, std::max(1, kAhead / u.bytes));
     u.ahead = std::min(kRecs, (kAhead + u.bytes - 1) / u.bytes);
     const int64_t parts = u.group > 1 ? (g.batch + u.group - 1) / u.group : g.batch * (u.mp * u.np);
-    rp.timeout_ns = (uint64_t)(2e9 + (double)g.num_iter * 1e6);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return launch_ring(rp, (int)std::min<int64_t>(parts, sms), s);
+    return (int)std::min<int64_t>(parts, sms);
+}
+
+// A uniform batch, A row-major and B N x K, M, N, K <= 128, 16-byte aligned
+// rows and problems (checked by the callers); KAMI_ERR_UNSUPPORTED, nothing
+// launched, where the strides exceed 32 bits.
+int f64_ring_launch(const GemmArgs &g, cudaStream_t s)
+{
+    if (g.lda > 0x7fffffff || g.ldb > 0x7fffffff || g.ldc > 0x7fffffff)
+        return fail(KAMI_ERR_UNSUPPORTED, "no kernel for M=%d N=%d K=%d with rows %lld, %lld, %lld apart", g.M, g.N, g.K,
+                    (long long)g.lda, (long long)g.ldb, (long long)g.ldc);
+    RingParams rp{};
+    rp.p.A = g.A;
+    rp.p.B = g.B;
+    rp.p.C = g.C;
+    rp.p.out_type = KAMI_F64;
+    rp.p.alpha = g.alpha;
+    rp.p.beta = g.beta;
+    rp.p.num_iter = g.num_iter;
+    rp.timeout_ns = (uint64_t)(2e9 + (double)g.num_iter * 1e6);
+    const int ctas = uniform_params(g, rp.u);
+    return launch_ring(rp, ctas, s);
+}
+
+// the launch of f64_ring_launch (kami_gemm_describe)
+void f64_ring_info(const GemmArgs &g, LaunchInfo *info)
+{
+    Uniform u{};
+    const int ctas = uniform_params(g, u);
+    *info = LaunchInfo{KAMI_VARIANT_MMA_SYNC, KAMI_PARTITION_1D, 1, kThreads, kSmem,
+                       ctas ? (int)((g.batch + ctas - 1) / ctas) : 0, ctas};
 }
 
 int f64_ring_read_error(int *flag)

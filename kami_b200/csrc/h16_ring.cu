@@ -607,6 +607,15 @@ int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, i
     return launch_ring(rp, bf16, ctas, s);
 }
 
+// CTAs of a uniform batch: one per SM, four problems side by side in each
+static int uniform_ctas(int64_t batch)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (int)std::min<int64_t>(batch, sms);
+}
+
 // A uniform batch, A row-major and B N x K, M, N, K <= 128, K a multiple of 8,
 // 16-byte aligned rows and problems (checked by the callers).
 int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s)
@@ -637,10 +646,15 @@ int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s)
     u.bytes = (up8(g.M) + up8(g.N)) * 128;
     u.slots = std::min(kRecs, kBytes / u.bytes);
     rp.timeout_ns = (uint64_t)(2e9 + (double)g.num_iter * 1e6);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return launch_ring(rp, in_type == KAMI_BF16, (int)std::min<int64_t>(g.batch, sms), s);
+    return launch_ring(rp, in_type == KAMI_BF16, uniform_ctas(g.batch), s);
+}
+
+// the launch of h16_ring_launch (kami_gemm_describe)
+void h16_ring_info(const GemmArgs &g, LaunchInfo *info)
+{
+    const int ctas = uniform_ctas(g.batch);
+    *info = LaunchInfo{KAMI_VARIANT_TCGEN05, KAMI_PARTITION_1D, 1, kThreads, kSmem,
+                       ctas ? (int)((g.batch + ctas - 1) / ctas) : 0, ctas};
 }
 
 int grouped_tc05_read_error(int *flag)

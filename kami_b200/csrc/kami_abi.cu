@@ -22,6 +22,8 @@ int split_read_error(int *flag);
 int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream);
 int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
 int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s);
+void f64_ring_info(const GemmArgs &g, LaunchInfo *info);
+void h16_ring_info(const GemmArgs &g, LaunchInfo *info);
 
 static thread_local char g_err[512] = "no error";
 
@@ -229,6 +231,52 @@ static bool aligned(const void *p, int64_t ld, int64_t s, int vec_elems, int esz
     return ((uintptr_t)p % (uintptr_t)(vec_elems * esz)) == 0 && ld % vec_elems == 0 && s % vec_elems == 0;
 }
 
+// Whether a uniform batch goes to the ring kernel of its type (f64_ring.cu,
+// h16_ring.cu): only where the choice is left to the library, up to four
+// repeats, A in rows and B as N x K.
+static bool ring_takes(int in_type, int partition, int variant, int P, int alloc_warps, const GemmArgs &g)
+{
+    if (variant != KAMI_VARIANT_AUTO || partition != KAMI_PARTITION_AUTO || P != 0 || alloc_warps != 0 ||
+        g.num_iter > 4 || g.a_layout != KAMI_A_ROW_MK || g.b_layout != KAMI_B_REF_NK || g.ldc > 0x7fffffff)
+        return false;
+    const int M = g.M, N = g.N, K = g.K, largest = std::max(M, std::max(N, K));
+    const double bytes = (double)g.batch * ((double)(M + N) * K * elem_size(in_type) +
+                                            (double)M * N * elem_size(g.out_type));
+    if (in_type == KAMI_F64)
+    {
+        // The per-problem kernel keeps what it holds in a compiled block
+        // without much padding and without a persistent kernel's start-up: up to
+        // 16^3 (400 MB of 16^3 58.6 us against 72, 2 MB of 8^3 2.2 against 3.6), and
+        // up to 32^3 below 32 MB or with strided rows (16 MB of 32^3 5.4 us against
+        // 6.3, 100 MB 24.6 against 21; strided, which the ring copies row by row,
+        // 150 MB 34 against 47).  Elsewhere the ring is ahead, from 1.1x at
+        // 64^3 to 5x where a 64^3 block is mostly padding (40 x 24 x 32).
+        const bool packed = (g.lda == K || M == 1) && (g.ldb == K || N == 1);
+        return largest <= 64 && g.lda <= 0x7fffffff && g.ldb <= 0x7fffffff &&
+               (largest > 32 || (largest > 16 && packed && bytes >= 32e6));
+    }
+    if (largest > 128 || K % 8 != 0 || g.lda > 0x3fffffff || g.ldb > 0x3fffffff || !aligned(g.A, g.lda, 0, 8, 2) ||
+        !aligned(g.B, g.ldb, 0, 8, 2) || (g.batch > 1 && (g.sA % 8 != 0 || g.sB % 8 != 0)))
+        return false;
+    // 16 bits: where the other kernels mostly pad (us below: FP16 in, FP32 out).
+    // The per-problem mma.sync kernel (M <= 32 or N < 32) keeps compiled sizes
+    // up to 16^3 (300 MB 60 against 160), and below 16 MB what fits 32^3 (4 MB of
+    // 32^3 3.2 against 4.6; 40 MB 25 against 14) and N that is not a multiple
+    // of 8, whose rows the ring stores in pieces (4 MB of 24 x 100 x 72 7.3
+    // against 12.6; 40 MB 70 against 34); elsewhere the ring is ahead, up to 11x
+    // (300 MB of 100 x 16 x 40 635 against 58, of 20 x 20 x 128 1073 against 94).
+    // The TMA kernels keep M > 64 (300 MB of 72 x 88 x 104 64 against 68, 128^3 54
+    // against 61), 64 rows of 64 columns or more (64^3 55 against 55 to 64),
+    // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
+    // 12.0 against 13.6) and N that is not a multiple of 8 (300 MB of
+    // 50 x 33 x 64 117 against 140); other blocks of up to 64 rows take the ring
+    // (48^3 84 against 55, 40^3 119 against 55, 64 x 40 x 64 67 against 55,
+    // 33 x 128 x 40 88 against 63).
+    if (tc05_prefer(in_type, partition, M, N, K, g.a_layout, g.b_layout))
+        return N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256;
+    return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0));
+}
+
 } // namespace kami
 
 using namespace kami;
@@ -333,8 +381,27 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type, kami_partiti
     if (st)
         return st;
     LaunchInfo info{};
-    if (variant == KAMI_VARIANT_TCGEN05 || variant == KAMI_VARIANT_TCGEN05_TS ||
-        (variant == KAMI_VARIANT_AUTO && tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout)))
+    GemmArgs g{}; // as packed and aligned as such a request can be
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.batch = batch;
+    g.a_layout = a_layout;
+    g.b_layout = b_layout;
+    g.lda = a_layout == KAMI_A_ROW_MK ? K : M;
+    g.ldb = b_layout == KAMI_B_REF_NK ? K : N;
+    g.ldc = N;
+    g.sA = (int64_t)M * K;
+    g.sB = (int64_t)N * K;
+    g.sC = (int64_t)M * N;
+    g.out_type = out_type;
+    g.alpha = 1.0;
+    g.num_iter = 1;
+    const bool ring = ring_takes(in_type, partition, variant, P, alloc_warps, g);
+    if (ring)
+        in_type == KAMI_F64 ? f64_ring_info(g, &info) : h16_ring_info(g, &info);
+    else if (variant == KAMI_VARIANT_TCGEN05 || variant == KAMI_VARIANT_TCGEN05_TS ||
+             (variant == KAMI_VARIANT_AUTO && tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout)))
     {
         const int ts = variant == KAMI_VARIANT_TCGEN05_TS ||
                        (variant == KAMI_VARIANT_AUTO && tc05_prefer_ts(M, a_layout));
@@ -342,7 +409,7 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type, kami_partiti
         if (st && variant != KAMI_VARIANT_AUTO)
             return st;
     }
-    if (info.variant != KAMI_VARIANT_TCGEN05 && info.variant != KAMI_VARIANT_TCGEN05_TS)
+    if (!ring && info.variant != KAMI_VARIANT_TCGEN05 && info.variant != KAMI_VARIANT_TCGEN05_TS)
     {
         const MmaInstance *inst = nullptr;
         st = plan_mma(in_type, partition, P, alloc_warps, M, N, K, batch, &inst, &info, false);
@@ -356,7 +423,7 @@ int kami_gemm_describe(kami_dtype_t in_type, kami_dtype_t out_type, kami_partiti
     out[4] = info.smem;
     out[5] = info.problems_per_cta;
     out[6] = (int)(info.grid > 0x7fffffff ? 0x7fffffff : info.grid);
-    out[7] = 0;
+    out[7] = ring;
     return KAMI_OK;
 }
 
@@ -433,35 +500,8 @@ int gemm_batched_hinted(kami_dtype_t in_type, kami_dtype_t out_type, kami_partit
     g.one_per_sm = one_per_sm;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
-    // Streamed 16-bit problems: the ring kernel, when the choice is left to the
-    // library, where the other kernels mostly pad (us below: FP16 in, FP32 out).
-    // The per-problem mma.sync kernel (M <= 32 or N < 32) keeps compiled sizes
-    // up to 16^3 (300 MB 60 against 160), and below 16 MB what fits 32^3 (4 MB of
-    // 32^3 3.2 against 4.6; 40 MB 25 against 14) and N that is not a multiple
-    // of 8, whose rows the ring stores in pieces (4 MB of 24 x 100 x 72 7.3
-    // against 12.6; 40 MB 70 against 34); elsewhere the ring is ahead, up to 11x
-    // (300 MB of 100 x 16 x 40 635 against 58, of 20 x 20 x 128 1073 against 94).
-    // The TMA kernels keep M > 64 (300 MB of 72 x 88 x 104 64 against 68, 128^3 54
-    // against 61), 64 rows of 64 columns or more (64^3 55 against 55 to 64),
-    // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
-    // 12.0 against 13.6) and N that is not a multiple of 8 (300 MB of
-    // 50 x 33 x 64 117 against 140); other blocks of up to 64 rows take the ring
-    // (48^3 84 against 55, 40^3 119 against 55, 64 x 40 x 64 67 against 55,
-    // 33 x 128 x 40 88 against 63).
-    if (in_type != KAMI_F64 && variant == KAMI_VARIANT_AUTO && partition == KAMI_PARTITION_AUTO && P == 0 &&
-        alloc_warps == 0 && num_iter <= 4 && M <= 128 && N <= 128 && K <= 128 && K % 8 == 0 &&
-        a_layout == KAMI_A_ROW_MK && b_layout == KAMI_B_REF_NK && !(reinterpret_cast<uintptr_t>(A) & 15) &&
-        !(reinterpret_cast<uintptr_t>(B) & 15) && lda % 8 == 0 && ldb % 8 == 0 &&
-        (batch == 1 || (strideA % 8 == 0 && strideB % 8 == 0)) && lda <= 0x3fffffff && ldb <= 0x3fffffff &&
-        ldc <= 0x7fffffff)
-    {
-        const int largest = std::max(M, std::max(N, K));
-        const double bytes = (double)batch * ((double)(M + N) * K * esz + (double)M * N * osz);
-        const bool tma = tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout);
-        if (tma ? N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256
-                : largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0)))
-            return h16_ring_launch(g, in_type, s);
-    }
+    if (ring_takes(in_type, partition, variant, P, alloc_warps, g))
+        return in_type == KAMI_F64 ? f64_ring_launch(g, s) : h16_ring_launch(g, in_type, s);
 
     if (variant == KAMI_VARIANT_TCGEN05 || variant == KAMI_VARIANT_TCGEN05_TS ||
         (variant == KAMI_VARIANT_AUTO && tc05_prefer(in_type, partition, M, N, K, a_layout, b_layout)))
@@ -471,25 +511,6 @@ int gemm_batched_hinted(kami_dtype_t in_type, kami_dtype_t out_type, kami_partit
         st = tc05_launch(g, in_type, partition, P, workspace, ws_bytes, s, ts);
         if (st == KAMI_OK || variant != KAMI_VARIANT_AUTO)
             return st;
-    }
-
-    // streamed FP64 problems: the ring kernel, when the choice is left to the
-    // library.  The per-problem kernel keeps what it holds in a compiled block
-    // without much padding and without a persistent kernel's start-up: up to
-    // 16^3 (400 MB of 16^3 58.6 us against 72, 2 MB of 8^3 2.2 against 3.6), and
-    // up to 32^3 below 32 MB or with strided rows (16 MB of 32^3 5.4 us against
-    // 6.3, 100 MB 24.6 against 21; strided, which the ring copies row by row,
-    // 150 MB 34 against 47).  Elsewhere the ring is ahead, from 1.1x at
-    // 64^3 to 5x where a 64^3 block is mostly padding (40 x 24 x 32).
-    if (in_type == KAMI_F64 && variant == KAMI_VARIANT_AUTO && partition == KAMI_PARTITION_AUTO && P == 0 &&
-        alloc_warps == 0 && num_iter <= 4 && M <= 64 && N <= 64 && K <= 64 && a_layout == KAMI_A_ROW_MK &&
-        b_layout == KAMI_B_REF_NK && lda <= 0x7fffffff && ldb <= 0x7fffffff && ldc <= 0x7fffffff)
-    {
-        const int largest = std::max(M, std::max(N, K));
-        const bool packed = (lda == K || M == 1) && (ldb == K || N == 1);
-        const double bytes = 8.0 * batch * ((double)(M + N) * K + (double)M * N);
-        if (largest > 32 || (largest > 16 && packed && bytes >= 32e6))
-            return f64_ring_launch(g, s);
     }
 
     const MmaInstance *inst = nullptr;
