@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "grouped.cuh"
@@ -95,9 +96,22 @@ struct Uniform
     int nk, bytes, slots; // chunks of a problem, ring bytes of one, chunks that a ring holds
 };
 
+// How C is written, by value: read from the kernel's parameters by reference, it
+// would be read again after every store, which for all the compiler knows has
+// changed it (1000 x 48 x 128 x 64, FP32 out, alpha 2, beta 0.5: 59 us, 21 so;
+// 4000 uneven problems of 8 .. 128, most of them of ragged N, 51 and 27).
+struct Out
+{
+    void *C;
+    int type;
+    bool plain, read; // alpha 1 and beta 0; beta not 0
+    float alpha, beta;
+};
+
 struct RingParams
 {
     GroupedParams p;
+    Out out; // from p
     const ChunkDesc *chunks; // a plan's chunks, null for a uniform batch
     Uniform u;
     uint64_t timeout_ns;
@@ -237,70 +251,128 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint4 (&v)[4])
                  : "memory");
 }
 
-// two neighbours of C (the first alone when cnt is 1) from x, y, with alpha /
-// beta and the output type
-__device__ __forceinline__ void store_two(const GroupedParams &p, bool plain, int64_t off, int cnt, float x, float y)
+// 16 rows x 16 columns of fragments v, of which rows x cols are the problem's, to
+// q: T is FP32's float or the 16-bit types' uint16_t, pairs: columns come in pairs
+// that may be read and stored at once.  C's old values are all asked for before the
+// first is used.
+template <class T>
+__device__ __forceinline__ void store_patch(const Out &o, const uint4 &v0, const uint4 &v1, T *q, int64_t down,
+                                            bool pairs, int rows, int cols)
 {
-    const float a = (float)p.alpha, b = (float)p.beta;
-    if (p.out_type == KAMI_F32)
+    const bool bf = o.type == KAMI_BF16;
+    const int lane = threadIdx.x & 31, gq = lane >> 2, c = 2 * (lane & 3);
+    // pair i: columns 8 (i / 2) + c and the next, of row gq or (odd i) gq + 8
+    float x[4][2] = {{__uint_as_float(v0.x), __uint_as_float(v0.y)}, {__uint_as_float(v0.z), __uint_as_float(v0.w)},
+                     {__uint_as_float(v1.x), __uint_as_float(v1.y)}, {__uint_as_float(v1.z), __uint_as_float(v1.w)}};
+    bool in0[4], in1[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
     {
-        float *q = reinterpret_cast<float *>(p.C) + off;
-        if (!plain)
+        in0[i] = gq + 8 * (i & 1) < rows && 4 * (i & 2) + c < cols;
+        in1[i] = in0[i] && 4 * (i & 2) + c + 1 < cols;
+    }
+    if (!o.plain)
+    {
+        // (as they lie in memory: unpacked at once, each load would be waited for)
+        using Word = std::conditional_t<sizeof(T) == 4, float2, uint32_t>;
+        Word word[4] = {};
+        T one[4][2] = {};
+        if (o.read && pairs)
         {
-            x = a * x + (p.beta != 0.0 ? b * q[0] : 0.f);
-            if (cnt > 1)
-                y = a * y + (p.beta != 0.0 ? b * q[1] : 0.f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (in0[i])
+                    word[i] = *reinterpret_cast<const Word *>(q + (i & 1) * down + 4 * (i & 2));
         }
-        if (cnt > 1 && !(reinterpret_cast<uintptr_t>(q) & 7))
-            *reinterpret_cast<float2 *>(q) = make_float2(x, y);
+        else if (o.read)
+        {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const T *w = q + (i & 1) * down + 4 * (i & 2);
+                one[i][0] = in0[i] ? w[0] : T(0);
+                one[i][1] = in1[i] ? w[1] : T(0);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            float y0, y1;
+            if constexpr (sizeof(T) == 4)
+            {
+                y0 = pairs ? word[i].x : one[i][0];
+                y1 = pairs ? word[i].y : one[i][1];
+            }
+            else
+            {
+                y0 = to_float(pairs ? (T)word[i] : one[i][0], bf);
+                y1 = to_float(pairs ? (T)(word[i] >> 16) : one[i][1], bf);
+            }
+            x[i][0] = o.alpha * x[i][0] + (o.read ? o.beta * y0 : 0.f);
+            x[i][1] = o.alpha * x[i][1] + (o.read ? o.beta * y1 : 0.f);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+        T *w = q + (i & 1) * down + 4 * (i & 2);
+        T y[2];
+        if constexpr (sizeof(T) == 4)
+            y[0] = x[i][0], y[1] = x[i][1];
         else
         {
-            q[0] = x;
-            if (cnt > 1)
-                q[1] = y;
+            const uint32_t h = pack2(x[i][0], x[i][1], bf);
+            y[0] = (T)h, y[1] = (T)(h >> 16);
         }
-        return;
-    }
-    const bool bf = p.out_type == KAMI_BF16;
-    uint16_t *q = reinterpret_cast<uint16_t *>(p.C) + off;
-    if (!plain)
-    {
-        x = a * x + (p.beta != 0.0 ? b * to_float(q[0], bf) : 0.f);
-        if (cnt > 1)
-            y = a * y + (p.beta != 0.0 ? b * to_float(q[1], bf) : 0.f);
-    }
-    const uint32_t h = pack2(x, y, bf);
-    if (cnt > 1 && !(reinterpret_cast<uintptr_t>(q) & 3))
-        *reinterpret_cast<uint32_t *>(q) = h;
-    else
-    {
-        q[0] = (uint16_t)h;
-        if (cnt > 1)
-            q[1] = (uint16_t)(h >> 16);
+        if (pairs)
+        {
+            if constexpr (sizeof(T) == 4)
+            {
+                if (in0[i])
+                    *reinterpret_cast<float2 *>(w) = make_float2(y[0], y[1]);
+            }
+            else if (in0[i])
+                *reinterpret_cast<ushort2 *>(w) = make_ushort2(y[0], y[1]);
+        }
+        else
+        {
+            if (in0[i])
+                w[0] = y[0];
+            if (in1[i])
+                w[1] = y[1];
+        }
     }
 }
 
-// Any other C: 16 rows x 32 columns of the accumulator at taddr, of which rows
-// x cols are the problem's, to off.  In fragment shape, so that a store covers
-// eight rows of up to 32 bytes however they are aligned (a row per lane would
-// spread it over 32 pieces).
-__device__ __noinline__ void store_general(const GroupedParams &p, uint32_t taddr, int64_t off, int64_t ldc, int rows,
-                                           int cols)
+// Any other C: `rows` rows of the accumulator's lanes at taddr, N columns, to off.
+// In fragment shape, so that a store covers eight rows of up to 32 bytes however
+// they are aligned (a row per lane would spread it over 32 pieces).
+__device__ __noinline__ void store_general(const Out &out, uint32_t taddr, int64_t off, int ldc, int rows, int N)
 {
-    const bool plain = p.alpha == 1.0 && p.beta == 0.0;
+    const Out o = out;
     const int lane = threadIdx.x & 31, gq = lane >> 2, c = 2 * (lane & 3);
-    uint4 v[4];
-    tmem_ld_frag32(taddr, v);
-    off += gq * ldc + c;
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-        if (8 * b + c < cols)
+    const int64_t down = 8 * (int64_t)ldc;
+    off += (int64_t)gq * ldc + c;
+    for (int h = 0; h < 32 && h < rows; h += 16)
+        for (int c0 = 0; c0 < N; c0 += 32)
         {
-            const int cnt = min(2, cols - 8 * b - c);
-            if (gq < rows)
-                store_two(p, plain, off + 8 * b, cnt, __uint_as_float(v[b].x), __uint_as_float(v[b].y));
-            if (gq + 8 < rows)
-                store_two(p, plain, off + 8 * ldc + 8 * b, cnt, __uint_as_float(v[b].z), __uint_as_float(v[b].w));
+            uint4 v[4];
+            tmem_ld_frag32(taddr + ((uint32_t)h << 16) + c0, v);
+            const int64_t at = off + (int64_t)h * ldc + c0;
+            if (o.type == KAMI_F32)
+            {
+                float *q = reinterpret_cast<float *>(o.C) + at;
+                const bool pairs = !((ldc | N) & 1) && !(reinterpret_cast<uintptr_t>(q) & 7); // the same in all lanes
+                store_patch(o, v[0], v[1], q, down, pairs, rows - h, N - c0);
+                store_patch(o, v[2], v[3], q + 16, down, pairs, rows - h, N - c0 - 16);
+            }
+            else
+            {
+                uint16_t *q = reinterpret_cast<uint16_t *>(o.C) + at;
+                const bool pairs = !((ldc | N) & 1) && !(reinterpret_cast<uintptr_t>(q) & 3);
+                store_patch(o, v[0], v[1], q, down, pairs, rows - h, N - c0);
+                store_patch(o, v[2], v[3], q + 16, down, pairs, rows - h, N - c0 - 16);
+            }
         }
 }
 
@@ -476,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
         __syncthreads();
         tc::tc_fence_after();
         const int q = warp & 3;
-        const bool plain = p.alpha == 1.0 && p.beta == 0.0;
+        const bool plain = rp.out.plain;
         const int own = rp.chunks ? p.cta_begin[workers + 1 + worker] : n / rp.u.nk; // problems
         for (int turn = 0; turn < own; ++turn)
         {
@@ -506,11 +578,8 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
                         store_row(p, off, N - c0, v);
                 }
             }
-            else
-                for (int h = base < 0 ? 32 : 0; h < 32 && base + h < M; h += 16)
-                    for (int c0 = 0; c0 < N; c0 += 32)
-                        store_general(p, lanes + ((uint32_t)h << 16) + c0,
-                                      r.c_off + (int64_t)(base + h) * r.ldc + c0, r.ldc, M - base - h, N - c0);
+            else if (base >= 0 && base < M)
+                store_general(rp.out, lanes, r.c_off + (int64_t)base * r.ldc, r.ldc, M - base, N);
             tc::tc_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -531,7 +600,7 @@ const void *ring_fn(bool bf16)
     return bf16 ? (const void *)&h16_ring_kernel<true> : (const void *)&h16_ring_kernel<false>;
 }
 
-int launch_ring(const RingParams &rp, bool bf16, int ctas, cudaStream_t s)
+int launch_ring(RingParams &rp, bool bf16, int ctas, cudaStream_t s)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -544,7 +613,9 @@ int launch_ring(const RingParams &rp, bool bf16, int ctas, cudaStream_t s)
     });
     if (attr[dev][bf16] != cudaSuccess)
         return cuda_fail(attr[dev][bf16], "cudaFuncSetAttribute(h16_ring_kernel)");
-    void *args[] = {const_cast<RingParams *>(&rp)};
+    rp.out = Out{rp.p.C, rp.p.out_type, rp.p.alpha == 1.0 && rp.p.beta == 0.0, rp.p.beta != 0.0, (float)rp.p.alpha,
+                 (float)rp.p.beta};
+    void *args[] = {&rp};
     e = launch_overlapped(ring_fn(bf16), dim3(ctas), dim3(kThreads), args, kSmem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(h16_ring_kernel)");
