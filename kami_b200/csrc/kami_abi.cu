@@ -247,10 +247,12 @@ static bool ring_takes(int in_type, int partition, int variant, int P, int alloc
         // The per-problem kernel keeps what it holds in a compiled block
         // without much padding and without a persistent kernel's start-up: up to
         // 16^3 (400 MB of 16^3 58.6 us against 72, 2 MB of 8^3 2.2 against 3.6), and
-        // up to 32^3 below 32 MB or with strided rows (16 MB of 32^3 5.4 us against
-        // 6.3, 100 MB 24.6 against 21; strided, which the ring copies row by row,
-        // 150 MB 34 against 47).  Elsewhere the ring is ahead, from 1.1x at
-        // 64^3 to 5x where a 64^3 block is mostly padding (40 x 24 x 32).
+        // up to 32^3 below 32 MB or with strided rows (24 MB of 32^3 6.0 us against
+        // 6.7, 197 MB 40 against 34; strided, which the ring copies row by row,
+        // 42 against 67).  Elsewhere the ring is ahead, packed (one 64^3 7.9 against
+        // 6.1, 8000 of them 249 against 151, 8000 of 40 x 24 x 32, where a 64^3 block is
+        // mostly padding, 198 against 42) and strided (7.9 against 6.9, 250 against 161,
+        // 199 against 70; equal at its least, 250 of 64^3).
         const bool packed = (g.lda == K || M == 1) && (g.ldb == K || N == 1);
         return largest <= 64 && g.lda <= 0x7fffffff && g.ldb <= 0x7fffffff &&
                (largest > 32 || (largest > 16 && packed && bytes >= 32e6));
@@ -258,22 +260,26 @@ static bool ring_takes(int in_type, int partition, int variant, int P, int alloc
     if (largest > 128 || K % 8 != 0 || g.lda > 0x3fffffff || g.ldb > 0x3fffffff || !aligned(g.A, g.lda, 0, 8, 2) ||
         !aligned(g.B, g.ldb, 0, 8, 2) || (g.batch > 1 && (g.sA % 8 != 0 || g.sB % 8 != 0)))
         return false;
-    // 16 bits: where the other kernels mostly pad (us below: FP16 in, FP32 out).
+    // 16 bits: where the other kernels mostly pad (us below: theirs / the ring's,
+    // FP16 in, FP32 out).
     // The per-problem mma.sync kernel (M <= 32 or N < 32) keeps compiled sizes
-    // up to 16^3 (300 MB 60 against 160), and below 16 MB what fits 32^3 (4 MB of
-    // 32^3 3.2 against 4.6; 40 MB 25 against 14) and N that is not a multiple
-    // of 8, whose rows the ring stores in pieces (4 MB of 24 x 100 x 72 7.3
-    // against 12.6; 40 MB 70 against 34); elsewhere the ring is ahead, up to 11x
-    // (300 MB of 100 x 16 x 40 635 against 58, of 20 x 20 x 128 1073 against 94).
-    // The TMA kernels keep M > 64 (300 MB of 72 x 88 x 104 64 against 68, 128^3 54
-    // against 61), 64 rows of 64 columns or more (64^3 55 against 55 to 64),
+    // up to 16^3 (300 MB 59 / 164), and below 16 MB what fits 32^3 (4 MB of 32^3
+    // 3.6 / 4.5; 40 MB 17.4 / 12.8) and N that is not a multiple of 8 (1 MB of
+    // 20 x 17 x 64 3.6 / 4.8, of 24 x 100 x 72 6.7 / 6.8; a line drawn when the ring
+    // stored such rows twice as slowly: 16 MB of the latter 24 / 8); elsewhere the
+    // ring is ahead, up to 15x (300 MB of 100 x 16 x 40 626 / 55, of 20 x 20 x 128
+    // 1061 / 69).
+    // The TMA kernels keep M > 64 (300 MB of 128^3 52 / 61; of 72 x 88 x 104 64 / 54),
+    // 64 rows of 64 columns or more (40 MB of 64^3 9.2 / 10.3, 300 MB 54.5 / 52.6),
     // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
-    // 12.0 against 13.6) and N that is not a multiple of 8 (300 MB of
-    // 50 x 33 x 64 117 against 140); other blocks of up to 64 rows take the ring
-    // (48^3 84 against 55, 40^3 119 against 55, 64 x 40 x 64 67 against 55,
-    // 33 x 128 x 40 88 against 63).
+    // 10.5 / 10.4), 16-bit C that is read (beta; 1000 of 48 x 128 x 64 23 / 27, of 48^3
+    // 12.5 / 13.6, of 64 x 56 x 64 16.6 / 14.9) and N that is not a multiple of 8 (from
+    // the same time: 300 MB of 50 x 33 x 64 117 / 140 then, 117 / 78 now); other blocks
+    // of up to 64 rows take the ring (300 MB of 48^3 85 / 55, of 40^3 120 / 51, of
+    // 64 x 40 x 64 68 / 53, of 33 x 128 x 40 87 / 65).
     if (tc05_prefer(in_type, partition, M, N, K, g.a_layout, g.b_layout))
-        return N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256;
+        return N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256 &&
+               (g.beta == 0.0 || g.out_type == KAMI_F32);
     return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0));
 }
 
