@@ -579,6 +579,18 @@ __global__ void spgemm_symbolic_lookback_kernel(int mb, int nb, const int *__res
 // ---------------------------------------------------------------------------
 // numeric
 // ---------------------------------------------------------------------------
+// How C is written: by value to push_store, which would read the kernel's
+// parameters again after each store otherwise, and ask for the second half of the
+// old tile only then (numeric pass with alpha and beta, 4096 rows of 6: 117 us, 84
+// so).
+struct PushOut
+{
+    void *vc;
+    int type;
+    bool read; // beta is not 0
+    float alpha, beta;
+};
+
 struct SpNumArgs
 {
     int mb, nb;
@@ -590,6 +602,7 @@ struct SpNumArgs
     int out_type;
     float alpha, beta;
     int num_iter;
+    PushOut push; // C as above
 };
 
 // Store one C tile with alpha / beta (lane layout of store_tile_frag).
@@ -887,43 +900,61 @@ constexpr int kFillWords = 512;   // FILL: words of 32 block columns
 
 // C tile c with alpha / beta in any output type: lane (gq, tq) holds columns
 // 4 tq .. 4 tq + 3 of rows gq (lo) and gq + 8 (hi).  beta == 0 never reads C.
-__device__ __noinline__ void push_store(const SpNumArgs &p, int64_t c, int gq, int tq, const float4 lo, const float4 hi)
+__device__ __noinline__ void push_store(const PushOut o, int64_t c, int gq, int tq, float4 lo, float4 hi)
 {
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
+    const int64_t at = c * 256 + gq * 16 + 4 * tq;
+    auto scale = [&](float4 &v, float4 was) {
+        v = make_float4(o.alpha * v.x + o.beta * was.x, o.alpha * v.y + o.beta * was.y, o.alpha * v.z + o.beta * was.z,
+                        o.alpha * v.w + o.beta * was.w);
+    };
+    if (o.type == KAMI_F32)
     {
-        const float4 v = h ? hi : lo;
-        const int at = (gq + 8 * h) * 16 + 4 * tq;
-        if (p.out_type == KAMI_F32)
+        float *const q = reinterpret_cast<float *>(o.vc) + at;
+        if (!(reinterpret_cast<uintptr_t>(o.vc) & 15))
         {
-            float2 *o = reinterpret_cast<float2 *>(reinterpret_cast<float *>(p.vc) + c * 256 + at);
-            float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
-            if (p.alpha != 1.f || p.beta != 0.f)
+            float4 *const p0 = reinterpret_cast<float4 *>(q), *const p1 = reinterpret_cast<float4 *>(q + 128);
+            if (o.alpha != 1.f || o.read)
             {
-                float2 q = make_float2(0.f, 0.f), r = q;
-                if (p.beta != 0.f)
-                    q = o[0], r = o[1];
-                x = make_float2(p.alpha * x.x + p.beta * q.x, p.alpha * x.y + p.beta * q.y);
-                y = make_float2(p.alpha * y.x + p.beta * r.x, p.alpha * y.y + p.beta * r.y);
+                float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f), w1 = w0;
+                if (o.read)
+                    w0 = *p0, w1 = *p1;
+                scale(lo, w0);
+                scale(hi, w1);
             }
-            o[0] = x;
-            o[1] = y;
+            *p0 = lo;
+            *p1 = hi;
+            return;
         }
-        else
+        float2 *const p0 = reinterpret_cast<float2 *>(q), *const p1 = reinterpret_cast<float2 *>(q + 128);
+        if (o.alpha != 1.f || o.read)
         {
-            uint2 *o = reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.vc) + c * 256 + at);
-            const bool bf = p.out_type == KAMI_BF16;
-            const uint2 old = p.beta != 0.f ? *o : make_uint2(0u, 0u);
-            auto cvt = [&](float f, uint32_t was) -> uint32_t {
-                float y = p.alpha * f;
-                if (p.beta != 0.f)
-                    y += p.beta * to_float((uint16_t)was, bf);
-                return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
-            };
-            *o = make_uint2(cvt(v.x, old.x & 0xffff) | (cvt(v.y, old.x >> 16) << 16),
-                            cvt(v.z, old.y & 0xffff) | (cvt(v.w, old.y >> 16) << 16));
+            float2 w00 = make_float2(0.f, 0.f), w01 = w00, w10 = w00, w11 = w00;
+            if (o.read)
+                w00 = p0[0], w01 = p0[1], w10 = p1[0], w11 = p1[1];
+            scale(lo, make_float4(w00.x, w00.y, w01.x, w01.y));
+            scale(hi, make_float4(w10.x, w10.y, w11.x, w11.y));
         }
+        p0[0] = make_float2(lo.x, lo.y);
+        p0[1] = make_float2(lo.z, lo.w);
+        p1[0] = make_float2(hi.x, hi.y);
+        p1[1] = make_float2(hi.z, hi.w);
+        return;
     }
+    uint2 *const p0 = reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(o.vc) + at), *const p1 = p0 + 32;
+    const bool bf = o.type == KAMI_BF16;
+    uint2 w0 = make_uint2(0u, 0u), w1 = w0;
+    if (o.read)
+        w0 = *p0, w1 = *p1;
+    auto cvt = [&](float f, uint32_t was) -> uint32_t {
+        float y = o.alpha * f;
+        if (o.read)
+            y += o.beta * to_float((uint16_t)was, bf);
+        return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
+    };
+    *p0 = make_uint2(cvt(lo.x, w0.x & 0xffff) | (cvt(lo.y, w0.x >> 16) << 16),
+                     cvt(lo.z, w0.y & 0xffff) | (cvt(lo.w, w0.y >> 16) << 16));
+    *p1 = make_uint2(cvt(hi.x, w1.x & 0xffff) | (cvt(hi.y, w1.x >> 16) << 16),
+                     cvt(hi.z, w1.y & 0xffff) | (cvt(hi.w, w1.y >> 16) << 16));
 }
 
 __device__ __forceinline__ uint32_t pack16(float x, float y, bool bf)
@@ -1181,7 +1212,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
         const int t = base + lane;
         unsigned none = __ballot_sync(0xffffffffu, t < t1 && sCnt[t] == (t ? sCnt[t - 1] : 0));
         for (; none; none &= none - 1)
-            push_store(p, c0 + base + __ffs(none) - 1, gq, tq, make_float4(0.f, 0.f, 0.f, 0.f),
+            push_store(p.push, c0 + base + __ffs(none) - 1, gq, tq, make_float4(0.f, 0.f, 0.f, 0.f),
                        make_float4(0.f, 0.f, 0.f, 0.f));
     }
     const uint32_t a_lane = tile_ldsm_addr((uint32_t)__cvta_generic_to_shared(sA), lane);
@@ -1249,7 +1280,7 @@ __global__ void __launch_bounds__(WARPS * 32) spgemm_numeric_push_kernel(const _
                             o[32] = make_uint2(pack16(hi.x, hi.y, bf), pack16(hi.z, hi.w, bf));
                         }
                         else
-                            push_store(p, c0 + (t & 0xffff), gq, tq, lo, hi);
+                            push_store(p.push, c0 + (t & 0xffff), gq, tq, lo, hi);
 #pragma unroll
                         for (int y = 0; y < 4; ++y)
                             acc0[y] = acc1[y] = 0.f;
@@ -1641,6 +1672,7 @@ static int numeric_pass(bool fill, kami_variant_t variant, kami_dtype_t in_type,
     p.alpha = (float)alpha;
     p.beta = (float)beta;
     p.num_iter = num_iter;
+    p.push = PushOut{val_c, out_type, p.beta != 0.f, p.alpha, p.beta};
     const int64_t grid = (nnz_c + 7) / 8;
     if (grid > 0x7fffffff)
         return fail(KAMI_ERR_UNSUPPORTED, "spgemm numeric: too many C tiles");
