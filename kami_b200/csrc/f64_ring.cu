@@ -561,6 +561,9 @@ size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *
     out->clear();
     out->reserve((problems + problems / 2) * sizeof(ChunkDesc));
     Placer placer(kRing);
+    // one shape's problems follow one another in a plan's order of cost: cut once
+    // (plan of 4000 128^3: 1.26 ms to create, 1.07 so)
+    int cut[3] = {0, 0, 0}, mb = 0, nb = 0;
     for (size_t c = 0; c < lists.size(); ++c)
     {
         (*begin)[c] = (int)count;
@@ -568,8 +571,8 @@ size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *
         int deal = 0;
         for (int i : lists[c])
         {
-            int mb = 0, nb = 0;
-            ring_cut(M[i], N[i], K[i], true, &mb, &nb);
+            if (M[i] != cut[0] || N[i] != cut[1] || K[i] != cut[2])
+                ring_cut(cut[0] = M[i], cut[1] = N[i], cut[2] = K[i], true, &mb, &nb);
             for (int r0 = 0; r0 < M[i]; r0 += mb)
                 for (int c0 = 0; c0 < N[i]; c0 += nb)
                 {
