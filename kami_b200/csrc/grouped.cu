@@ -464,6 +464,7 @@ struct kami_grouped_plan
     int in_type, out_type, count, ctas, smem;
     int kernel = 0; // 0: mma.sync warp grids (grouped_kernel), 1: tcgen05 (h16_ring_kernel),
                     // 2: FP64 ring (f64_ring_kernel)
+    int groups = 1; // tcgen05 plans: problem lists of a CTA
     int tc_m64 = 0, tc_m128 = 0; // tcgen05 plans: problems on M = 64 / M = 128 MMAs
     int small_begin = 0, small_end = 0; // desc range of single-warp problems
     void *d_desc = nullptr; // GroupedDesc per problem; the ring kernels' own descriptors
@@ -551,7 +552,7 @@ static int launch_grouped(const kami_grouped_plan *plan, const void *A, const vo
     p.small_begin = plan->small_begin;
     p.small_end = plan->small_end;
     if (plan->kernel == 1)
-        return grouped_tc05_launch(p, plan->d_desc, plan->in_type == KAMI_BF16, plan->ctas, s);
+        return grouped_tc05_launch(p, plan->d_desc, plan->in_type == KAMI_BF16, plan->ctas, plan->groups, s);
     if (plan->kernel == 2)
         return grouped_f64s_launch(p, plan->d_desc, plan->ctas, s);
     void *args[] = {&p};
@@ -602,7 +603,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     }
     occ = std::max(occ, 1);
     // tcgen05 plans have several lists of problems per CTA
-    const int per_cta = tc ? grouped_tc05_lists() : 1;
+    const int per_cta = tc ? grouped_tc05_lists(count, M, N) : 1;
     const int ctas = std::max(1, std::min(count, sms * occ)), nlists = ctas * per_cta;
     const int esz = in_type == KAMI_F64 ? 8 : 2;
     const int osz = out_type == KAMI_F64 ? 8 : out_type == KAMI_F32 ? 4 : 2;
@@ -615,6 +616,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     pl->out_type = out_type;
     pl->count = count;
     pl->ctas = ctas;
+    pl->groups = per_cta;
     pl->smem = smem;
     pl->kernel = kernel;
     std::vector<double> cost(count);
@@ -672,7 +674,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     if (staged)
         f64_ring_schedule(lists, M, N, K, ao, bo, co, &chunks, &begin);
     else if (tc)
-        h16_ring_schedule(lists, M, N, K, ao, bo, co, lda, ldb, ldc, &chunks, &begin);
+        h16_ring_schedule(lists, M, N, K, ao, bo, co, lda, ldb, ldc, &chunks, &begin, per_cta);
     const void *src = kernel ? (const void *)chunks.data() : (const void *)desc.data();
     const size_t src_bytes = kernel ? chunks.size() : sizeof(GroupedDesc) * desc.size();
     if ((e = cudaMalloc(&pl->d_desc, std::max(src_bytes, (size_t)16))) != cudaSuccess ||

@@ -6,7 +6,7 @@
 // what counts is how few instructions and hand-offs each one takes and how many
 // are on their way at once.  One CTA per SM runs four independent groups, each
 // with its own list of problems, its own ring of shared memory (ring.cuh, 46 KB)
-// and 128 columns of tensor memory:
+// and 128 columns of tensor memory (plans of large problems: two groups, with 92 KB):
 //   warps 20 + 2 g, 21 + 2 g copy A's and B's rows by 16-byte cp.async straight
 //               into the 128-byte-swizzled K-major layout the MMA reads (row r
 //               at r * 128, 16-byte chunk c at c ^ (r % 8)), 64 values of K to
@@ -409,7 +409,7 @@ __device__ __forceinline__ void store_row(const GroupedParams &p, int64_t off, i
         }
 }
 
-template <bool BF16>
+template <bool BF16, int GROUPS>
 __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_constant__ RingParams rp)
 {
     const GroupedParams &p = rp.p;
@@ -423,7 +423,11 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t limit = rp.timeout_ns;
     // this warp's group and what belongs to it
-    const int g = warp < kIssue ? warp >> 2 : warp < kCopy ? warp - kIssue : (warp - kCopy) >> 1;
+    // (two: groups 0 and 1 work, and the storing warps of 2 and 3 take every other
+    // problem of 0 and 1, out of accumulators of their own)
+    static_assert(GROUPS == kGroups || GROUPS == kGroups / 2, "groups at work");
+    constexpr bool two = GROUPS < kGroups;
+    const int g = warp < kIssue ? (warp >> 2) & (GROUPS - 1) : warp < kCopy ? warp - kIssue : (warp - kCopy) >> 1;
     Rec *recs = recs_all + g * kRecs, *grec = grec_all + 2 * g;
     uint64_t *full = bars + g * (2 * kRecs + 5);
     uint64_t *empty = full + kRecs;
@@ -453,21 +457,21 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
     }
     wait_for_previous();
     // the group's chunks: a plan's list, or every so many-th problem of the batch
-    const int worker = g * gridDim.x + blockIdx.x, workers = gridDim.x * kGroups;
-    int64_t first;
-    int n;
-    if (rp.chunks)
+    const int worker = g * gridDim.x + blockIdx.x, workers = gridDim.x * GROUPS;
+    int64_t first = 0;
+    int n = 0;
+    if (rp.chunks && (!two || g < GROUPS))
     {
         first = p.cta_begin[worker];
         n = p.cta_begin[worker + 1] - (int)first;
     }
-    else
+    else if (!two || g < GROUPS)
     {
         first = worker;
         n = worker < rp.u.batch ? (int)((rp.u.batch - worker + workers - 1) / workers) * rp.u.nk : 0;
     }
     if (warp >= kCopy)
-        copy_chunks(rp, tc::smem_u32(smem) + kFront + g * kBytes, recs, full, empty, first, n, workers, (warp - kCopy) & 1,
+        copy_chunks(rp, tc::smem_u32(smem) + kFront + g * (kBytes * kGroups / GROUPS), recs, full, empty, first, n, workers, (warp - kCopy) & 1,
                     lane);
     else if (warp >= kIssue)
     {
@@ -476,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
         tc::tc_fence_after();
         if (lane == 0)
         {
-            const uint32_t acc = *tmem_slot + g * 128;
+            const uint32_t acc = *tmem_slot + g * 128, apart = two ? 256 : 64;
             int turn = 0;        // problems so far
             bool wide = false;   // the current or last one takes all columns
             uint32_t idesc = 0, d = 0, more = 0, up = 0;
@@ -494,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
                 {
                     // the accumulator's last product (and, where one of the two
                     // takes all columns, the problem before) has been read out
-                    const bool now = N > 64;
+                    const bool now = N > 64 && !two;
                     if ((turn >= 2 && !tc::mbar_wait_bounded(&acce[b], ((turn >> 1) - 1) & 1, limit)) ||
                         (turn >= 1 && (now || wide) &&
                          !tc::mbar_wait_bounded(&acce[b ^ 1], ((turn - 1) >> 1) & 1, limit)))
@@ -510,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
                     c.quad = quad;
                     grec[b] = c;
                     idesc = tc::idesc_f16(BF16, 128, (N + 15) & ~15);
-                    d = acc + (now ? 0 : 64 * b);
+                    d = acc + (now ? 0 : apart * b);
                     more = 0;
                 }
                 // the copies are generic-proxy writes: order them before the
@@ -550,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
         const int q = warp & 3;
         const bool plain = rp.out.plain;
         const int own = rp.chunks ? p.cta_begin[workers + 1 + worker] : n / rp.u.nk; // problems
-        for (int turn = 0; turn < own; ++turn)
+        for (int turn = two ? warp >> 3 : 0; turn < own; turn += two ? 2 : 1)
         {
             const int b = turn & 1;
             // (tcgen05.ld is .sync.aligned: the outcome must be warp-uniform)
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
             tc::tc_fence_after();
             const Rec r = grec[b];
             const int M = r.shape & 255, N = (r.shape >> 8) & 255;
-            const uint32_t acc = *tmem_slot + g * 128 + (N > 64 ? 0 : 64 * b);
+            const uint32_t acc = *tmem_slot + g * 128 + (two ? 256 * b : N > 64 ? 0 : 64 * b);
             const int base = 32 * (q - r.quad); // the row in this warp's first lane
             const bool fast = plain && !((r.ldc | (int)r.c_off | N) & 7) && !(reinterpret_cast<uintptr_t>(p.C) & 31);
             const uint32_t lanes = acc + ((uint32_t)(32 * q) << 16);
@@ -595,28 +599,33 @@ __global__ void __launch_bounds__(kThreads, 1) h16_ring_kernel(const __grid_cons
     }
 }
 
-const void *ring_fn(bool bf16)
+const void *ring_fn(bool bf16, bool two)
 {
-    return bf16 ? (const void *)&h16_ring_kernel<true> : (const void *)&h16_ring_kernel<false>;
+    if (two)
+        return bf16 ? (const void *)&h16_ring_kernel<true, kGroups / 2> : (const void *)&h16_ring_kernel<false, kGroups / 2>;
+    return bf16 ? (const void *)&h16_ring_kernel<true, kGroups> : (const void *)&h16_ring_kernel<false, kGroups>;
 }
 
-int launch_ring(RingParams &rp, bool bf16, int ctas, cudaStream_t s)
+int launch_ring(RingParams &rp, bool bf16, int groups, int ctas, cudaStream_t s)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev >= 64)
         return e != cudaSuccess ? cuda_fail(e, "cudaGetDevice") : KAMI_ERR_UNSUPPORTED;
-    static std::once_flag once[64][2];
-    static cudaError_t attr[64][2];
-    std::call_once(once[dev][bf16], [&] {
-        attr[dev][bf16] = cudaFuncSetAttribute(ring_fn(bf16), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    static std::once_flag once[64][4];
+    static cudaError_t attr[64][4];
+    const bool two = groups < kGroups;
+    const void *fn = ring_fn(bf16, two);
+    const int v = bf16 + 2 * two;
+    std::call_once(once[dev][v], [&] {
+        attr[dev][v] = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     });
-    if (attr[dev][bf16] != cudaSuccess)
-        return cuda_fail(attr[dev][bf16], "cudaFuncSetAttribute(h16_ring_kernel)");
+    if (attr[dev][v] != cudaSuccess)
+        return cuda_fail(attr[dev][v], "cudaFuncSetAttribute(h16_ring_kernel)");
     rp.out = Out{rp.p.C, rp.p.out_type, rp.p.alpha == 1.0 && rp.p.beta == 0.0, rp.p.beta != 0.0, (float)rp.p.alpha,
                  (float)rp.p.beta};
     void *args[] = {&rp};
-    e = launch_overlapped(ring_fn(bf16), dim3(ctas), dim3(kThreads), args, kSmem, s);
+    e = launch_overlapped(fn, dim3(ctas), dim3(kThreads), args, kSmem, s);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaLaunchKernel(h16_ring_kernel)");
     return KAMI_OK;
@@ -625,7 +634,25 @@ int launch_ring(RingParams &rp, bool bf16, int ctas, cudaStream_t s)
 } // namespace
 
 int grouped_tc05_smem() { return kSmem; }
-int grouped_tc05_lists() { return kGroups; }
+// Groups at work in a plan's CTAs.  A group's 46 KB hold one chunk of a large
+// problem, which its MMAs have to be done with before the next is copied: where
+// problems of more than half a ring carry most of the bytes, two groups of 92 KB
+// (us, four groups / two: 2000 of 128^3 55 / 52, 4000 with FP16 out 80 / 71, 2000 of
+// 96^3 34 / 28, 1000 of 112 .. 128 25 / 23; the other way at times, 4000 of 112 .. 128
+// 84 / 90).  All sixteen storing warps stay at work: half of them, 1000 of 128^3
+// with alpha and beta took 62 us instead of 45.  (A kernel of its own: the same
+// choice at run time cost 20000 of 32^3 9 %.)
+int grouped_tc05_lists(int count, const int *M, const int *N)
+{
+    int64_t all = 0, large = 0;
+    for (int i = 0; i < count; ++i)
+    {
+        const int bytes = (up8(M[i]) + up8(N[i])) * 128;
+        all += bytes;
+        large += 2 * bytes > kBytes ? bytes : 0;
+    }
+    return 2 * large > all ? kGroups / 2 : kGroups;
+}
 
 // The problems of a plan's lists, one per group (list l: group l / CTAs of CTA
 // l % CTAs, so that few problems spread over the CTAs first), as chunks
@@ -633,7 +660,7 @@ int grouped_tc05_lists() { return kGroups; }
 // lists + 1 on) their numbers of problems.
 void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
                        const int64_t *ao, const int64_t *bo, const int64_t *co, const int *lda, const int *ldb,
-                       const int *ldc, std::vector<char> *out, std::vector<int> *begin)
+                       const int *ldc, std::vector<char> *out, std::vector<int> *begin, int groups)
 {
     size_t count = 0, total = 0;
     for (const auto &l : lists)
@@ -642,7 +669,7 @@ void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M,
     out->resize(total * sizeof(ChunkDesc));
     begin->assign(2 * lists.size() + 1, 0);
     ChunkDesc *d = reinterpret_cast<ChunkDesc *>(out->data());
-    ring::Placer placer(kBytes, kRecs);
+    ring::Placer placer(kBytes * kGroups / groups, kRecs);
     for (size_t c = 0; c < lists.size(); ++c)
     {
         (*begin)[c] = (int)count;
@@ -669,13 +696,13 @@ void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M,
 }
 
 // a plan: descriptors (h16_ring_schedule) on the device, p.cta_begin their lists
-int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, cudaStream_t s)
+int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, int groups, cudaStream_t s)
 {
     RingParams rp{};
     rp.p = p;
     rp.chunks = reinterpret_cast<const ChunkDesc *>(chunks);
     rp.timeout_ns = (uint64_t)(2e9 + (double)p.num_iter * 1e6); // generous: a problem takes microseconds
-    return launch_ring(rp, bf16, ctas, s);
+    return launch_ring(rp, bf16, groups, ctas, s);
 }
 
 // CTAs of a uniform batch: one per SM, four problems side by side in each
@@ -717,7 +744,7 @@ int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s)
     u.bytes = (up8(g.M) + up8(g.N)) * 128;
     u.slots = std::min(kRecs, kBytes / u.bytes);
     rp.timeout_ns = (uint64_t)(2e9 + (double)g.num_iter * 1e6);
-    return launch_ring(rp, in_type == KAMI_BF16, uniform_ctas(g.batch), s);
+    return launch_ring(rp, in_type == KAMI_BF16, kGroups, uniform_ctas(g.batch), s);
 }
 
 // the launch of h16_ring_launch (kami_gemm_describe)
