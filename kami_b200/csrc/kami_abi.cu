@@ -263,12 +263,14 @@ static bool ring_takes(int in_type, int partition, int variant, int P, int alloc
     // 16 bits: where the other kernels mostly pad (us below: theirs / the ring's,
     // FP16 in, FP32 out).
     // The per-problem mma.sync kernel (M <= 32 or N < 32) keeps compiled sizes
-    // up to 16^3 (300 MB 59 / 164), and below 16 MB what fits 32^3 (4 MB of 32^3
-    // 3.6 / 4.5; 40 MB 17.4 / 12.8) and N that is not a multiple of 8 (1 MB of
-    // 20 x 17 x 64 3.6 / 4.8, of 24 x 100 x 72 6.7 / 6.8; a line drawn when the ring
-    // stored such rows twice as slowly: 16 MB of the latter 24 / 8); elsewhere the
-    // ring is ahead, up to 15x (300 MB of 100 x 16 x 40 626 / 55, of 20 x 20 x 128
-    // 1061 / 69).
+    // up to 16^3 (300 MB 59 / 164), what fits 64^3 up to two problems per SM, which
+    // it has all at once (in a graph, 100 of 8 x 40 x 40 2.2 / 3.4, of 32 x 64 x 64
+    // 2.8 / 3.5, 300 of them 3.2 / 3.5 and 4.1 / 4.2, 450 4.3 / 3.8 and 5.6 / 4.8), and
+    // below 16 MB what fits 32^3 (4 MB of 32^3 3.6 / 4.5; 40 MB 17.4 / 12.8) and N
+    // that is not a multiple of 8 (1 MB of 20 x 17 x 64 3.6 / 4.8, of 24 x 100 x 72
+    // 6.7 / 6.8; a line drawn when the ring stored such rows twice as slowly: 16 MB of
+    // the latter 24 / 8); elsewhere the ring is ahead, up to 15x (300 MB of
+    // 100 x 16 x 40 626 / 55, of 20 x 20 x 128 1061 / 69).
     // The TMA kernels keep M > 64 (300 MB of 128^3 52 / 61; of 72 x 88 x 104 64 / 54),
     // 64 rows of 64 columns or more (40 MB of 64^3 9.2 / 10.3, 300 MB 54.5 / 52.6),
     // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
@@ -280,7 +282,7 @@ static bool ring_takes(int in_type, int partition, int variant, int P, int alloc
     if (tc05_prefer(in_type, partition, M, N, K, g.a_layout, g.b_layout))
         return N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256 &&
                (g.beta == 0.0 || g.out_type == KAMI_F32);
-    return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0));
+    return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0 && (largest > 64 || g.batch > 296)));
 }
 
 } // namespace kami

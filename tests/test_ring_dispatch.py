@@ -20,8 +20,10 @@ def _describe(dtype, M, N, K, batch, variant=_lib.VARIANT_AUTO, partition=_lib.P
 
 
 RING = [(_lib.F16, 40, 40, 40, 100), (_lib.BF16, 100, 16, 40, 10), (_lib.F16, 20, 20, 128, 1600),
-        (_lib.F16, 33, 128, 40, 1), (_lib.F64, 64, 64, 64, 5), (_lib.F64, 40, 24, 32, 1), (_lib.F64, 32, 32, 32, 2000)]
+        (_lib.F16, 33, 128, 40, 1), (_lib.F16, 32, 64, 64, 300), (_lib.F64, 64, 64, 64, 5),
+        (_lib.F64, 40, 24, 32, 1), (_lib.F64, 32, 32, 32, 2000)]
 OTHER = [(_lib.F16, 128, 128, 128, 592), (_lib.F16, 16, 16, 16, 10 ** 6), (_lib.F16, 20, 20, 128, 900),
+         (_lib.F16, 32, 64, 64, 296), (_lib.BF16, 8, 40, 40, 1),
          (_lib.F16, 33, 41, 128, 1500), (_lib.F64, 16, 16, 16, 10 ** 5), (_lib.F64, 32, 32, 32, 1000)]
 
 
