@@ -274,15 +274,19 @@ static bool ring_takes(int in_type, int partition, int variant, int P, int alloc
     // The TMA kernels keep M > 64 (300 MB of 128^3 52 / 61; of 72 x 88 x 104 64 / 54),
     // 64 rows of 64 columns or more (40 MB of 64^3 9.2 / 10.3, 300 MB 54.5 / 52.6),
     // problems of which a group's ring holds only one (40 MB of 48 x 128 x 96
-    // 10.5 / 10.4), 16-bit C that is read (beta; 1000 of 48 x 128 x 64 23 / 27, of 48^3
-    // 12.5 / 13.6, of 64 x 56 x 64 16.6 / 14.9) and N that is not a multiple of 8 (from
-    // the same time: 300 MB of 50 x 33 x 64 117 / 140 then, 117 / 78 now); other blocks
-    // of up to 64 rows take the ring (300 MB of 48^3 85 / 55, of 40^3 120 / 51, of
-    // 64 x 40 x 64 68 / 53, of 33 x 128 x 40 87 / 65).
+    // 10.5 / 10.4), C with alpha or beta where N > 64 or problems are few or C is of 16
+    // bits and read (in a graph, 4000 of 48 x 128 x 64 40 / 47, 100 of 48^3 4.7 / 5.4,
+    // 1000 of 48 x 128 x 64 with beta 23 / 27; 4000 of 48^3 24 / 19; the mma.sync kernel
+    // likewise, 100 of 16 x 104 x 40 4.7 / 5.5) and N that is not a multiple of 8 (a
+    // line from the same time: 300 MB of 50 x 33 x 64 117 / 140 then, 117 / 78 now);
+    // other blocks of up to 64 rows take the ring (300 MB of 48^3 85 / 55, of 40^3
+    // 120 / 51, of 64 x 40 x 64 68 / 53, of 33 x 128 x 40 87 / 65).
+    const bool few = g.batch <= 296, scaled = g.alpha != 1.0 || g.beta != 0.0;
     if (tc05_prefer(in_type, partition, M, N, K, g.a_layout, g.b_layout))
         return N % 8 == 0 && M <= 64 && (M < 64 || N < 64) && (M + N) * ((K + 63) / 64) <= 256 &&
-               (g.beta == 0.0 || g.out_type == KAMI_F32);
-    return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0 && (largest > 64 || g.batch > 296)));
+               (!scaled || (N <= 64 && !few && (g.beta == 0.0 || g.out_type == KAMI_F32)));
+    return largest > 16 && (bytes >= 16e6 || (largest > 32 && N % 8 == 0 &&
+                                              (!few || (largest > 64 && !(scaled && N > 64)))));
 }
 
 } // namespace kami
