@@ -126,11 +126,16 @@ struct Operand
 
 void *entries(const Tensor &t) { return t.numel() ? t.data_ptr() : nullptr; }
 
+// Calls f without the interpreter lock, and holds it again however f ends: what
+// catches an exception needs it.
 template <class F> int unlocked(F &&f)
 {
-    int st;
-    Py_BEGIN_ALLOW_THREADS st = f();
-    Py_END_ALLOW_THREADS return st;
+    struct Unlock
+    {
+        PyThreadState *const state = PyEval_SaveThread();
+        ~Unlock() { PyEval_RestoreThread(state); }
+    } unlock;
+    return f();
 }
 
 // Runs f: a tensor (or tuple) object, or a status, or NotImplemented.
