@@ -509,7 +509,7 @@ int launch_ring(const RingParams &rp, int ctas, cudaStream_t s)
 
 } // namespace
 
-int grouped_f64s_smem() { return kSmem; }
+int f64_ring_smem() { return kSmem; }
 
 // Cut of an M x N problem into parts of mb x nb (multiples of 16 unless whole)
 // with at most a tile for each computing warp: the one that reads the fewest
@@ -612,7 +612,7 @@ size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *
 }
 
 // a plan: chunks (f64_ring_schedule) on the device, p.cta_begin their lists
-int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s)
+int f64_ring_plan_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s)
 {
     RingParams rp{};
     rp.p = p;

@@ -552,9 +552,9 @@ static int launch_grouped(const kami_grouped_plan *plan, const void *A, const vo
     p.small_begin = plan->small_begin;
     p.small_end = plan->small_end;
     if (plan->kernel == 1)
-        return grouped_tc05_launch(p, plan->d_desc, plan->in_type == KAMI_BF16, plan->ctas, plan->groups, s);
+        return h16_ring_plan_launch(p, plan->d_desc, plan->in_type == KAMI_BF16, plan->ctas, plan->groups, s);
     if (plan->kernel == 2)
-        return grouped_f64s_launch(p, plan->d_desc, plan->ctas, s);
+        return f64_ring_plan_launch(p, plan->d_desc, plan->ctas, s);
     void *args[] = {&p};
     cudaError_t e = cudaLaunchKernel(grouped_fn(plan->in_type), dim3(plan->ctas), dim3(kThreads), args,
                                      (size_t)plan->smem, s);
@@ -582,8 +582,7 @@ static int free_plan(kami_grouped_plan *pl)
 // kernel's cost model is its bytes plus a fixed per-problem latency.
 static int build_plan(int in_type, int out_type, int count, const int *M, const int *N, const int *K,
                       const int64_t *ao, const int64_t *bo, const int64_t *co, const int *cfg,
-                      kami_grouped_plan **out, const int *lda = nullptr, const int *ldb = nullptr,
-                      const int *ldc = nullptr, int kernel = 0)
+                      kami_grouped_plan **out, int kernel = 0)
 {
     int dev = 0, sms = 0, occ = 0;
     cudaError_t e;
@@ -592,7 +591,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return cuda_fail(e, "cudaDeviceGetAttribute");
     const bool tc = kernel == 1, staged = kernel == 2;
-    const int smem = tc ? grouped_tc05_smem() : staged ? grouped_f64s_smem() : grouped_smem(in_type);
+    const int smem = tc ? h16_ring_smem() : staged ? f64_ring_smem() : grouped_smem(in_type);
     if (!tc && !staged) // (the ring kernels run one CTA per SM)
     {
         const void *fn = grouped_fn(in_type);
@@ -603,7 +602,7 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     }
     occ = std::max(occ, 1);
     // tcgen05 plans have several lists of problems per CTA
-    const int per_cta = tc ? grouped_tc05_lists(count, M, N) : 1;
+    const int per_cta = tc ? h16_ring_groups(count, M, N) : 1;
     const int ctas = std::max(1, std::min(count, sms * occ)), nlists = ctas * per_cta;
     const int esz = in_type == KAMI_F64 ? 8 : 2;
     const int osz = out_type == KAMI_F64 ? 8 : out_type == KAMI_F32 ? 4 : 2;
@@ -660,21 +659,19 @@ static int build_plan(int in_type, int out_type, int count, const int *M, const 
     {
         begin[c] = (int)desc.size();
         for (int i : lists[c])
-            desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], lda ? lda[i] : K[i],
-                                       ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i]});
+            desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], K[i], K[i], N[i]});
     }
     begin[ctas] = (int)desc.size();
     pl->small_begin = (int)desc.size();
     for (int i : smalls)
-        desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], lda ? lda[i] : K[i],
-                                   ldb ? ldb[i] : K[i], ldc ? ldc[i] : N[i]});
+        desc.push_back(GroupedDesc{M[i], N[i], K[i], cfg[i], ao[i], bo[i], co[i], K[i], K[i], N[i]});
     pl->small_end = (int)desc.size();
     // ring plans: the kernels' own descriptors instead
     std::vector<char> chunks;
     if (staged)
         f64_ring_schedule(lists, M, N, K, ao, bo, co, &chunks, &begin);
     else if (tc)
-        h16_ring_schedule(lists, M, N, K, ao, bo, co, lda, ldb, ldc, &chunks, &begin, per_cta);
+        h16_ring_schedule(lists, M, N, K, ao, bo, co, &chunks, &begin, per_cta);
     const void *src = kernel ? (const void *)chunks.data() : (const void *)desc.data();
     const size_t src_bytes = kernel ? chunks.size() : sizeof(GroupedDesc) * desc.size();
     if ((e = cudaMalloc(&pl->d_desc, std::max(src_bytes, (size_t)16))) != cudaSuccess ||
@@ -751,57 +748,20 @@ static int tune_shape(int in_type, int out_type, int M, int N, int K, void *A, v
 
 namespace kami {
 
-// Serve a batched request that no compiled block instance covers (e.g. FP64
-// above 64^3) with the grouped kernel: one plan per distinct request shape,
-// cached (descriptors hold offsets, not pointers, so a plan serves any
-// buffers).
+// Serve a batched request that no compiled block instance covers: FP64 above
+// 64^3, with the ring kernel (16-bit instances cover every size up to 128^3).
 int grouped_fallback(const GemmArgs &g, int in_type, cudaStream_t stream)
 {
     if (g.a_layout != KAMI_A_ROW_MK || g.b_layout != KAMI_B_REF_NK)
         return fail(KAMI_ERR_UNSUPPORTED, "no kernel for this shape with these layouts");
-    const int q = in_type == KAMI_F64 ? 2 : 8;
-    if (g.M > 128 || g.N > 128 || g.K > 128 || g.K % q || g.lda % q || g.ldb % q || g.sA % q || g.sB % q ||
-        g.batch > 1000000)
+    if (in_type != KAMI_F64 || g.M > 128 || g.N > 128 || g.K > 128 || g.K % 2 || g.lda % 2 || g.ldb % 2 || g.sA % 2 ||
+        g.sB % 2 || g.batch > 1000000)
         return fail(KAMI_ERR_UNSUPPORTED, "no kernel for M=%d N=%d K=%d (lda=%lld ldb=%lld)", g.M, g.N, g.K,
                     (long long)g.lda, (long long)g.ldb);
     if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.B) & 15) ||
         (reinterpret_cast<uintptr_t>(g.C) & 15))
         return fail(KAMI_ERR_UNSUPPORTED, "no kernel for this shape with unaligned buffers");
-    if (in_type == KAMI_F64)
-        return f64_ring_launch(g, stream);
-    static std::mutex mu;
-    static std::map<std::vector<int64_t>, kami_grouped_plan *> cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::vector<int64_t> key = {dev, in_type, g.out_type, g.M, g.N, g.K, g.batch, g.lda, g.ldb, g.ldc, g.sA, g.sB, g.sC};
-    kami_grouped_plan *pl = nullptr;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = cache.find(key);
-        if (it != cache.end())
-            pl = it->second;
-    }
-    if (!pl)
-    {
-        const int n = (int)g.batch;
-        std::vector<int> vm(n, g.M), vn(n, g.N), vk(n, g.K), vc(n, cfg_heuristic(in_type, g.M, g.N, g.K));
-        std::vector<int> la(n, (int)g.lda), lb(n, (int)g.ldb), lc(n, (int)g.ldc);
-        std::vector<int64_t> ao(n), bo(n), co(n);
-        for (int i = 0; i < n; ++i)
-        {
-            ao[i] = (int64_t)i * g.sA;
-            bo[i] = (int64_t)i * g.sB;
-            co[i] = (int64_t)i * g.sC;
-        }
-        int st = build_plan(in_type, g.out_type, n, vm.data(), vn.data(), vk.data(), ao.data(), bo.data(), co.data(),
-                            vc.data(), &pl, la.data(), lb.data(), lc.data(), 1);
-        if (st)
-            return st;
-        std::lock_guard<std::mutex> lk(mu);
-        if (cache.size() < 256)
-            cache[key] = pl;
-    }
-    return launch_grouped(pl, g.A, g.B, g.C, g.alpha, g.beta, g.num_iter, stream);
+    return f64_ring_launch(g, stream);
 }
 
 } // namespace kami
@@ -943,14 +903,14 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
         return build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), plan);
     if (force_tc || force_st || !tune || count == 0)
         return build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), plan,
-                          nullptr, nullptr, nullptr, alt);
+                          alt);
     // autotuned, kernel not forced: build both kernels' plans, time each on
     // scratch buffers of the plan's extent, keep the faster
     kami_grouped_plan *pl[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; ++k)
     {
         int st = build_plan(in_type, out_type, count, M, N, K, a_offsets, b_offsets, c_offsets, cfg.data(), &pl[k],
-                            nullptr, nullptr, nullptr, k == 0 ? 0 : alt);
+                            k == 0 ? 0 : alt);
         if (st)
         {
             free_plan(pl[0]);

@@ -33,21 +33,21 @@ struct GroupedParams
 
 // 16-bit ring kernel (h16_ring.cu): plans, and uniform batches
 // (h16_ring_launch)
-int grouped_tc05_smem();
-int grouped_tc05_lists(int count, const int *M, const int *N); // problem lists of a CTA
+int h16_ring_smem();
+int h16_ring_groups(int count, const int *M, const int *N); // problem lists of a CTA
 void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
-                       const int64_t *ao, const int64_t *bo, const int64_t *co, const int *lda, const int *ldb,
-                       const int *ldc, std::vector<char> *out, std::vector<int> *begin, int groups);
-int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, int groups, cudaStream_t s);
+                       const int64_t *ao, const int64_t *bo, const int64_t *co, std::vector<char> *out,
+                       std::vector<int> *begin, int groups);
+int h16_ring_plan_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, int groups, cudaStream_t s);
 int h16_ring_launch(const GemmArgs &g, int in_type, cudaStream_t s);
-int grouped_tc05_read_error(int *flag);
+int h16_ring_read_error(int *flag);
 
 // FP64 ring kernel (f64_ring.cu): plans, and uniform batches (f64_ring_launch)
-int grouped_f64s_smem();
+int f64_ring_smem();
 size_t f64_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
                          const int64_t *ao, const int64_t *bo, const int64_t *co, std::vector<char> *out,
                          std::vector<int> *begin);
-int grouped_f64s_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s);
+int f64_ring_plan_launch(const GroupedParams &p, const void *chunks, int ctas, cudaStream_t s);
 int f64_ring_launch(const GemmArgs &g, cudaStream_t s);
 int f64_ring_read_error(int *flag);
 

@@ -633,7 +633,7 @@ int launch_ring(RingParams &rp, bool bf16, int groups, int ctas, cudaStream_t s)
 
 } // namespace
 
-int grouped_tc05_smem() { return kSmem; }
+int h16_ring_smem() { return kSmem; }
 // Groups at work in a plan's CTAs.  A group's 46 KB hold one chunk of a large
 // problem, which its MMAs have to be done with before the next is copied: where
 // problems of more than half a ring carry most of the bytes, two groups of 92 KB
@@ -642,7 +642,7 @@ int grouped_tc05_smem() { return kSmem; }
 // 84 / 90).  All sixteen storing warps stay at work: half of them, 1000 of 128^3
 // with alpha and beta took 62 us instead of 45.  (A kernel of its own: the same
 // choice at run time cost 20000 of 32^3 9 %.)
-int grouped_tc05_lists(int count, const int *M, const int *N)
+int h16_ring_groups(int count, const int *M, const int *N)
 {
     int64_t all = 0, large = 0;
     for (int i = 0; i < count; ++i)
@@ -659,8 +659,8 @@ int grouped_tc05_lists(int count, const int *M, const int *N)
 // placed in the groups' rings.  begin: the lists' first chunks, then (from
 // lists + 1 on) their numbers of problems.
 void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M, const int *N, const int *K,
-                       const int64_t *ao, const int64_t *bo, const int64_t *co, const int *lda, const int *ldb,
-                       const int *ldc, std::vector<char> *out, std::vector<int> *begin, int groups)
+                       const int64_t *ao, const int64_t *bo, const int64_t *co, std::vector<char> *out,
+                       std::vector<int> *begin, int groups)
 {
     size_t count = 0, total = 0;
     for (const auto &l : lists)
@@ -686,9 +686,9 @@ void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M,
                 x.shape = (uint32_t)(M[i] | N[i] << 8 | std::min(64, K[i] - k0) << 16) | (k0 == 0 ? kFirst : 0u) |
                           (k0 + 64 >= K[i] ? kLast : 0u);
                 x.at = placer.place((up8(M[i]) + up8(N[i])) * 128, &x.dep, &land);
-                x.lda = lda ? lda[i] : K[i];
-                x.ldb = ldb ? ldb[i] : K[i];
-                x.ldc = ldc ? ldc[i] : N[i];
+                x.lda = K[i];
+                x.ldb = K[i];
+                x.ldc = N[i];
                 d[count++] = x;
             }
     }
@@ -696,7 +696,7 @@ void h16_ring_schedule(const std::vector<std::vector<int>> &lists, const int *M,
 }
 
 // a plan: descriptors (h16_ring_schedule) on the device, p.cta_begin their lists
-int grouped_tc05_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, int groups, cudaStream_t s)
+int h16_ring_plan_launch(const GroupedParams &p, const void *chunks, bool bf16, int ctas, int groups, cudaStream_t s)
 {
     RingParams rp{};
     rp.p = p;
@@ -755,7 +755,7 @@ void h16_ring_info(const GemmArgs &g, LaunchInfo *info)
                        ctas ? (int)((g.batch + ctas - 1) / ctas) : 0, ctas};
 }
 
-int grouped_tc05_read_error(int *flag)
+int h16_ring_read_error(int *flag)
 {
     int v = 0, z = 0;
     cudaError_t e = cudaMemcpyFromSymbol(&v, g_h16r_error, sizeof(int));

@@ -13,7 +13,7 @@
 
 namespace kami {
 
-int grouped_tc05_read_error(int *flag);
+int h16_ring_read_error(int *flag);
 int spgemm_read_error(int *flag);
 int f64_ring_read_error(int *flag);
 int spmm_tc05_read_error(int *flag);
@@ -316,7 +316,7 @@ int kami_device_status(int *code)
     int c2 = 0, c4 = 0, c5 = 0, c6 = 0, c7 = 0;
     if ((st = split_read_error(&c2)))
         return st;
-    if ((st = grouped_tc05_read_error(&c4)))
+    if ((st = h16_ring_read_error(&c4)))
         return st;
     if ((st = spgemm_read_error(&c5)))
         return st;
