@@ -440,8 +440,8 @@ int kami_spgemm_bsr_block(kami_dtype_t in_type, kami_dtype_t out_type, kami_part
                           double alpha, double beta, int num_iter, void *stream);
 
 /* kami_spgemm_bsr_numeric with the kernel chosen: KAMI_VARIANT_MMA_SYNC
- * (one CTA per block-row: A tiles staged, each C tile's products found by
- * searching its column in the B rows, two m16n8k16 MMAs per product),
+ * (one CTA per block-row: A tiles staged, the row's products enumerated once
+ * and grouped by C tile, two m16n8k16 MMAs per product),
  * KAMI_VARIANT_TCGEN05 (one CTA per SM: the row's products enumerated once
  * and streamed through a shared-memory ring, one tcgen05.mma of M = 64,
  * N = 16 per product into the tile's own tensor-memory accumulator; tile

@@ -17,8 +17,9 @@ returned in the input dtype, as torch.bmm does.
 
 The default path (the library's kernel choice) is the C++ operator
 torch.ops.kami.bmm (kami_b200/torch_ops/kami_torch_ops.cpp): the same two
-launches with its forward, backward node and argument handling in C++, so
-the host time per step stays below the kernels' time.
+launches with its forward, backward node and argument handling in C++.  The
+host time still decides a step of small heads: 62 us at BF16 4096 x 64^3, whose
+two kernels take 53.
 """
 from __future__ import annotations
 

@@ -883,9 +883,10 @@ int kami_gemm_grouped_plan_create(kami_dtype_t in_type, kami_dtype_t out_type, i
     const int alt = in_type == KAMI_F64 ? 2 : 1;
     // FP64 without a measurement: the ring kernel, except that a plan of less
     // than 10 MB with most of its bytes in problems of at most 32 x 32 keeps the
-    // warp-grid kernel it has always reported (measured, the ring is ahead from
-    // 1000 problems on: 1000 of 8..32 5.0 against 7.4 us, 20000 of 32^3 78
-    // against 146; 1000 of 8^3 4.5 against 4.0)
+    // warp-grid kernel it has always reported.  (It is not the faster one there: us in
+    // a graph, warp grids / ring, 300 of 32^3 8.6 / 3.7, 1000 of 8..32 9.2 / 5.3, 100 of
+    // 16^3 4.6 / 2.5, equal at 1000 of 8^3; above the line 2000 of 8..32 12.9 / 7.7.  A
+    // caller who wants the ring there asks for KAMI_PLAN_STAGED or KAMI_PLAN_AUTOTUNE.)
     bool tiny_mix = false;
     if (in_type == KAMI_F64 && !force_st && !tune)
     {

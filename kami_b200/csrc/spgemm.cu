@@ -19,13 +19,15 @@
 //     bitmap in shared memory (shared atomics), counts it with popc, and the
 //     column fill walks the bitmap words in order (ascending by
 //     construction);  the scan is a single-CTA in-place scan; no scratch.
-//   * numeric: one warp per C tile (i, j).  Its lanes take the nonzero
-//     blocks A(i, k) of row i, binary-search j in block-row k of B (column
-//     indices sorted ascending, as the reference generator emits them), and
-//     the warp accumulates every matching A(i,k) * B(k,j) with two
-//     m16n8k16 MMAs (FP32 accumulation) in ascending k -- the order of the
-//     reference's sparse accumulator.  No C tile is touched twice, so the
-//     kernel writes C once (the HBM floor of the product).
+//   * numeric: one CTA per block-row of C enumerates the row's products once,
+//     groups them by C tile, and its warps take the tiles in turn, each
+//     accumulating its products A(i,k) * B(k,j) with two m16n8k16 MMAs (FP32
+//     accumulation) in ascending k -- the order of the reference's sparse
+//     accumulator.  The column fill can ride along.  No C tile is touched twice,
+//     so the kernel writes C once (the HBM floor of the product).  Rows beyond
+//     what a CTA stages search each tile's products (column indices sorted
+//     ascending, as the reference generator emits them), and so does a warp per
+//     C tile where the tile arrays are not 16-byte aligned.
 #include <atomic>
 #include <cstdint>
 #include <mutex>

@@ -4,8 +4,8 @@
 //
 // A Python torch.autograd.Function spends tens of microseconds of host time
 // per step (the Python apply, two ctypes calls with their argument checks,
-// the autograd node); at 4096 x 64^3 the forward and the fused backward
-// kernels take ~75 us together, so that host time decides the step.  Here
+// the autograd node), 90 us at BF16 4096 x 64^3, whose forward and fused
+// backward kernels take 53 us together.  Here (62 us a step)
 // the forward, the backward node and both launches are C++: torch's
 // dispatcher calls kami_gemm_batched (forward, B as the K x N operand) and
 // kami_gemm_backward_batched (dA = dC B^T and dB = A^T dC in one fused
